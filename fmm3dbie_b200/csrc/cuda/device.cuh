@@ -87,6 +87,7 @@ struct MatvecArgs {
   int weff_f32 = 0;
   int far_variant = 0;            // far-kernel block shape (see far_block_targets)
   const void* ab = nullptr;       // per-source constants for the multi-density kernel
+  float* tc_ops = nullptr;        // tensor-core far field: its density operand (far_tc_operand_floats)
   int* tc_err = nullptr;          // set by the tensor-core far field if a completion wait timed out
   const int32_t* sdest = nullptr; // strengths: source s is stored at position sdest[s]
 };
@@ -130,6 +131,8 @@ int far_variants();
 // Helmholtz path): densities per CTA, 0 where the variant does not apply.
 int far_tc_group(int variant, int nd, int precision, int kind);
 int far_tc_targets();  // targets per CTA
+// Floats of a.tc_ops that every variant of (nd, precision, kind) fits in.
+size_t far_tc_operand_floats(int nd, int precision, int kind, int64_t nptso);
 // Launches it, or with occ != null reports its resident CTAs per SM.
 cudaError_t far_tc(int variant, const Geometry& g, const KParams& kp, const MatvecArgs& a,
                    cudaStream_t st, int* occ);

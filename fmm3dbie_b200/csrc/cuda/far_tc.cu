@@ -3,34 +3,57 @@
 // For nd densities the far field is, per target t and density m,
 //   y(t, m) = sum_s K(t, s) sigma(s, m),
 // a product of the kernel matrix with the density matrix.  Each CTA takes
-// 128 targets, one source chunk and N densities.  Per tile of 32 sources its
-// 512 threads evaluate the 128 x 32 kernel values with the same FP32 pair
-// function and block centring as the CUDA-core kernels (so the
-// error-matched W_eff32 fold still cancels their near-pair values) and lay
-// the complex product out as one real GEMM of M = 128 rows (targets),
-// K = 64 (kernel real parts, then imaginary parts) and 2N columns (the
-// densities' real parts, then their imaginary parts):
-//   A = [Kr | Ki],  B = [[sr, si], [-si, sr]],  Y = A B = [Re y | Im y].
-// Both operands are split into high and low parts (x = hi + lo, hi rounded
-// to TF32, lo rounded to TF32 as well) and one thread issues tcgen05.mma
-// kind::tf32 for hi*hi + hi*lo + lo*hi (the 3xTF32 scheme, about FP32
-// accuracy) into an FP32 accumulator of 2N columns in tensor memory, which
-// is read with tcgen05.ld after every tile and added into compensated
-// (Kahan) FP32 sums in registers;
-// the partial sums of the chunk are written in the CUDA-core kernels'
-// layout.  While the tensor core works on a tile, the threads load the next
-// tile's sources and densities into registers.  (Double-buffering the kernel
-// values and the accumulator, so that a tile's kernel values are computed
-// while the previous tile's MMAs run, measured slower: the kernel-value
-// stage, not the tensor core, sets the pace.)  Operands sit in shared
-// memory in the canonical no-swizzle K-major layout (8-row x 16-byte core
-// matrices, row groups 128 B apart, K-direction core matrices (rows / 8) x
-// 128 B apart).  Completion waits are bounded; on timeout the kernel records
-// the CTA in *err, waits once more (bounded) for its tensor-core work, frees
-// its tensor memory and writes nothing.
+// 128 targets, one source chunk and N densities and walks the chunk in tiles
+// of 64 sources.  With K = Kr + i Ki and sigma = sr + i si (scaled by the
+// source's weight / 4 pi) a tile adds
+//   Re y += Kr sr - Ki si,   Im y += Kr si + Ki sr,
+// formed as the two real products Kr [sr | si] and Ki [sr | si] in separate
+// accumulators (one B operand for both, every MMA 2 N columns wide) and put
+// together when they are read.  Every operand is split into high and low
+// parts (x = hi + lo, both read as TF32), and the products lo*hi, hi*lo,
+// hi*hi are issued in that order as tcgen05.mma kind::tf32 with FP32
+// accumulators in tensor memory (the 3xTF32 scheme): an accumulator rounds
+// after every K = 8 step, so the small products go in while it is small and
+// only its last steps round at full size.
+//
+// The kernel values go from the registers that computed them straight into
+// tensor memory (tcgen05.st, operand A); the density operand B is scaled,
+// split and laid out once per matvec by far_tc_operand_kernel in the
+// canonical no-swizzle K-major layout (8-row x 16-byte core matrices, row
+// groups 128 B apart, K-direction core matrices (2 N / 8) x 128 B apart) and
+// arrives by one bulk copy per tile.
+//
+// 18 warps per CTA, ordered only by mbarriers:
+//   warps 0-15  kernel values (warp w: targets 32 (w % 4) .. + 31, one per
+//               lane, sources 16 (w / 4) .. + 15 of the tile, two per packed
+//               instruction) with the FP32 pair arithmetic and block centring
+//               of the CUDA-core kernels, so that the error-matched W_eff32
+//               fold still cancels their near-pair values; and the sums: each
+//               thread adds N / 2 columns of its target into FP32 registers
+//               after every tile and every kTcFold tiles into FP64 ones;
+//   warp 16     producer: bulk copy of B, the tile's source coordinates;
+//   warp 17     issues the MMAs (the warp runs uniformly, one elected lane
+//               issues: from a single-lane branch the operands had to be
+//               moved to uniform registers for each MMA, which took 9.3
+//               instead of 5.7 ms at 16 densities).
+// While the tensor core works on a tile the SIMT warps evaluate the next.
+//
+// Measured (matvec of a 36,504-node surface with 77,974 oversampled nodes,
+// B200): 64 densities 17.3 -> 7.7 ms, 32: 15.5 -> 5.7, 16: 11.9 (CUDA cores)
+// -> 5.3, 4: 6.0 (CUDA cores) -> 5.0, against FP64 6.3e-7 (9.2e-7 before) at
+// 64 densities and 5.0e-7 (5.0e-7) at 16.  What bounds it: at 64 densities
+// the 48 MMAs of a tile (about 104 cycles each; 64 would be the tensor peak),
+// below that the kernel values with the operand splits (about 25 instructions
+// a pair; evaluation alone takes 3.4 of the 4.5 ms at 16 densities).
+//
+// Completion waits are bounded; on timeout the kernel records the CTA in
+// *err, every role leaves, the copies and MMAs in flight are waited for
+// (bounded), the tensor memory is freed and nothing is written.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "device.cuh"
 #include "pair.cuh"
@@ -40,116 +63,222 @@ namespace bie {
 namespace dev {
 namespace {
 
-constexpr int kTcT = 128;                     // targets per CTA = accumulator rows
-constexpr int kTcRows = kTcT;
-constexpr int kTcS = 32;                      // sources per tile
-constexpr int kTcK = 2 * kTcS;                // reduction length of a tile
-constexpr int kTcThreads = 512;
-constexpr uint32_t kTcLboA = (kTcRows / 8) * 128;
+constexpr int kTcT = 128;          // targets per CTA = accumulator rows
+constexpr int kTcS = 64;           // sources per tile
+constexpr int kTcWarps = 16;       // warps that evaluate kernel values
+constexpr int kTcThreads = 32 * (kTcWarps + 2);
+constexpr int kTcPer = kTcS * 4 / kTcWarps;  // sources of a tile per thread
+constexpr int kTcStages = 3;       // source tiles in flight
+constexpr int kTcFold = 8;         // tiles summed in the first set of registers
+constexpr int kTcACols = 4 * kTcS; // tensor-memory columns of A: Kr hi, Ki hi, Kr lo, Ki lo
+constexpr uint32_t kTcTmemCols = 512;
+
+// Parts a tile's sources are split into for N densities: each part has its own
+// two accumulators (Kr and Ki) of 2 N columns, so that an accumulator rounds
+// at full size in 8 / parts hi*hi steps.  As many as tensor memory holds at 16
+// densities (against FP64 on a 3,750-node sphere: 1.1e-7 with 4 parts, 2.4e-7
+// with 1; the CUDA-core kernel 1.14e-7).
+template <int N>
+constexpr int kTcSplit = N == 64 ? 1 : (N == 32 ? 2 : 4);
+
+constexpr uint32_t kTcSpin = 1u << 22;  // polls of one wait before the CTA gives up
+constexpr double kTcOver4Pi = 0.07957747154594767;
 static_assert(kFarTileSources % kTcS == 0, "chunks are whole tiles");
 
-// Compensated (Kahan) FP32 sum s + v: the running error sits in c, so the
-// sum stays accurate to about FP32 rounding over the whole chunk without
-// FP32-to-FP64 conversions (which would load the XU pipe).
-__device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
-  const float y = v - c;
-  const float t = s + y;
-  c = (t - s) - y;
-  s = t;
-}
-
-// (acc, cmp)[n] += accumulator row 32 (w % 4) + lane, columns c0 .. c0 + NH - 1
-// (a warp may read only the tensor-memory lanes of its quarter, w % 4).
-template <int NH>
-__device__ __forceinline__ void flush(uint32_t tmem, int c0, float* acc, float* cmp) {
-  const int quarter = (threadIdx.x >> 5) & 3;
-  const uint32_t lanes = uint32_t(quarter * 32) << 16;
-  if constexpr (NH == 8) {
-    uint32_t v[8];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-          "=r"(v[7])
-        : "r"(tmem + lanes + uint32_t(c0)));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int j = 0; j < 8; ++j) kahan_add(acc[j], cmp[j], __uint_as_float(v[j]));
-  } else {
-#pragma unroll
-    for (int cc = 0; cc < NH; cc += 16) {
-      uint32_t v[16];
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,"
-          "%13,%14,%15}, [%16];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-            "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
-            "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-          : "r"(tmem + lanes + uint32_t(c0 + cc)));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int j = 0; j < 16; ++j) kahan_add(acc[cc + j], cmp[cc + j], __uint_as_float(v[j]));
-    }
-  }
-}
-
-// Operands of one source tile held in registers while the previous tile's
-// MMAs run: the source (thread < 32) and this thread's density tasks.
+// Floats of one tile's B operand (hi part, then lo part): 2 N rows (real
+// parts, then imaginary parts of the densities) by kTcS sources.
 template <int N>
-struct TileRegs {
-  static constexpr int kTasks = (N * (kTcS / 4) + kTcThreads - 1) / kTcThreads;
-  double sx, sy, sz, nx, ny, nz;
-  float4 abv;
-  float2 sig[kTasks][4];
+constexpr int kTcOpFloats = 2 * 2 * N * kTcS;
+
+// One tile's sources: coordinates negated and centred, normals.
+struct TcGeom {
+  float x[kTcS], y[kTcS], z[kTcS], nx[kTcS], ny[kTcS], nz[kTcS];
+  int check, pad[3];
 };
 
 template <int N>
-__device__ __forceinline__ void tile_load(const Geometry& g, const float* __restrict__ ab,
-                                          const float* __restrict__ sig, int nd, int m0,
-                                          int64_t sb, int ns, TileRegs<N>& r) {
-  const int tid = threadIdx.x;
-  if (tid < kTcS) {
-    if (tid < ns) {
-      const int64_t s = sb + tid;
-      r.sx = g.sx[s], r.sy = g.sy[s], r.sz = g.sz[s];
-      r.nx = g.snx[s], r.ny = g.sny[s], r.nz = g.snz[s];
-      r.abv = *reinterpret_cast<const float4*>(ab + 4 * s);
+struct TcSmem {
+  float b[kTcStages][kTcOpFloats<N>];
+  TcGeom geom[kTcStages];
+  uint64_t full[kTcStages], empty[kTcStages], afull, done;
+  uint32_t tmem;
+  int fail;
+};
+
+// Waits (bounded) for phase `parity` of the barrier; false once any role of
+// the CTA has given up.
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
+  for (uint32_t it = 0; it < kTcSpin; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (*fail) return false;
+  }
+  *fail = 1;
+  return false;
+}
+
+// The same for a whole warp, one answer for all lanes.
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail) {
+  return __all_sync(0xffffffffu, tc_wait(bar, parity, fail));
+}
+
+__device__ __forceinline__ void tc_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Kernel values K = alpha G + beta dG/dn of one target against two sources
+// (lane .x and lane .y): per lane the operations of pair_helm.
+// Constants of the kernel values, each twice (the two lanes); a kernel
+// parameter, so that they stay in the constant bank.
+struct TcConst {
+  float2 k, kim, ar, ai, br, bi, mbr, one, mone;
+  float thr2;
+};
+
+template <bool CHECK, bool CK>
+__device__ __forceinline__ void tc_pair(const float2 tx, const float2 ty, const float2 tz,
+                                        const float2 msx, const float2 msy, const float2 msz,
+                                        const float2 nx, const float2 ny, const float2 nz,
+                                        const TcConst& c, float2& kr_, float2& ki_) {
+  const float2 dx = __fadd2_rn(tx, msx), dy = __fadd2_rn(ty, msy), dz = __fadd2_rn(tz, msz);
+  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+  float2 rinv;
+  rinv.x = (!CHECK || r2.x >= c.thr2) ? rsqrtf(r2.x) : 0.0f;
+  rinv.y = (!CHECK || r2.y >= c.thr2) ? rsqrtf(r2.y) : 0.0f;
+  const float2 r = __fmul2_rn(r2, rinv);
+  const float2 kr = __fmul2_rn(c.k, r);
+  float2 sn, cs;
+  __sincosf(kr.x, &sn.x, &cs.x);
+  __sincosf(kr.y, &sn.y, &cs.y);
+  float2 rs = rinv;
+  if (CK) {
+    rs.x *= __expf(-c.kim.x * r.x);
+    rs.y *= __expf(-c.kim.y * r.y);
+  }
+  const float2 dn = __ffma2_rn(dx, nx, __ffma2_rn(dy, ny, __fmul2_rn(dz, nz)));
+  const float2 u = __fmul2_rn(dn, __fmul2_rn(rinv, rinv));
+  float2 xr, xi;
+  if (CK) {
+    const float2 ur = __fmul2_rn(u, __ffma2_rn(c.kim, r, c.one));
+    const float2 p = __fmul2_rn(u, kr);
+    xr = __ffma2_rn(c.bi, p, __ffma2_rn(c.br, ur, c.ar));
+    xi = __ffma2_rn(c.mbr, p, __ffma2_rn(c.bi, ur, c.ai));
+  } else {
+    xr = __ffma2_rn(u, __ffma2_rn(c.bi, kr, c.br), c.ar);
+    xi = __ffma2_rn(u, __ffma2_rn(c.mbr, kr, c.bi), c.ai);
+  }
+  const float2 er = __fmul2_rn(xr, rs), ei = __fmul2_rn(xi, rs);
+  const float2 msn = __fmul2_rn(sn, c.mone);
+  kr_ = __ffma2_rn(cs, er, __fmul2_rn(msn, ei));
+  ki_ = __ffma2_rn(cs, ei, __fmul2_rn(sn, er));
+}
+
+__device__ __forceinline__ void tmem_store16(uint32_t addr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,"
+      "%14,%15,%16};" ::"r"(addr),
+      "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]),
+      "f"(v[8]), "f"(v[9]), "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+      : "memory");
+}
+
+// x -> high part (rounded to TF32) and remainder, which the tensor core reads
+// as TF32 (of its 12 significant bits at most the last one goes).
+__device__ __forceinline__ void split_store16(uint32_t hi_addr, uint32_t lo_addr, float* v) {
+  float hi[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    hi[j] = tf32_rn(v[j]);
+    v[j] -= hi[j];
+  }
+  tmem_store16(hi_addr, hi);
+  tmem_store16(lo_addr, v);
+}
+
+__device__ __forceinline__ void tmem_load8(uint32_t addr, float* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
+                 "=f"(v[6]), "=f"(v[7])
+               : "r"(addr));
+}
+
+// sum[n] += column c0 + n of Kr [sr | si] + i Ki [sr | si] from the tile's
+// accumulators (this warp's lane quarter), two columns per packed operation:
+// real parts Kr sr - Ki si, imaginary parts Kr si + Ki sr.
+template <int N, int NH, int SPLIT>
+__device__ __forceinline__ void flush_add(uint32_t tmem, int c0, float2* sum) {
+  const bool re = c0 < N;
+  const int ci = re ? c0 + N : c0 - N;
+  const float2 sg = re ? make_float2(-1.f, -1.f) : make_float2(1.f, 1.f);
+#pragma unroll
+  for (int c = 0; c < NH; c += 8) {
+    float v[SPLIT][2][8];
+#pragma unroll
+    for (int h = 0; h < SPLIT; ++h) {
+      tmem_load8(tmem + uint32_t(h * 4 * N + c0 + c), v[h][0]);
+      tmem_load8(tmem + uint32_t(h * 4 * N + 2 * N + ci + c), v[h][1]);
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float2 t[SPLIT];
+#pragma unroll
+      for (int h = 0; h < SPLIT; ++h)
+        t[h] = __ffma2_rn(sg, make_float2(v[h][1][j], v[h][1][j + 1]),
+                          make_float2(v[h][0][j], v[h][0][j + 1]));
+      if constexpr (SPLIT >= 2) t[0] = __fadd2_rn(t[0], t[1]);
+      if constexpr (SPLIT == 4) t[0] = __fadd2_rn(t[0], __fadd2_rn(t[2], t[3]));
+      sum[(c + j) / 2] = __fadd2_rn(sum[(c + j) / 2], t[0]);
     }
   }
-#pragma unroll
-  for (int k = 0; k < TileRegs<N>::kTasks; ++k) {
-    const int q = tid + k * kTcThreads;
-    const int n = q % N, sq = 4 * (q / N), m = m0 + n;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      r.sig[k][u] = make_float2(0.f, 0.f);
-      if (q < N * (kTcS / 4) && sq + u < ns && m < nd)
-        r.sig[k][u] = *reinterpret_cast<const float2*>(sig + (size_t(sb + sq + u) * nd + m) * 2);
-    }
-  }
+}
+
+template <bool ACC>
+__device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(d),
+      "r"(a), "l"(b), "r"(idesc), "n"(ACC ? 1 : 0)
+      : "memory");
+}
+
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void tc_commit(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+          smem_u32(bar))
+      : "memory");
 }
 
 template <int N, bool CK>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    far_tc_kernel(Geometry g, KParams kp, const float* __restrict__ ab,
-                  const float* __restrict__ sig, int nd, double* __restrict__ partial,
-                  int64_t chunk_len, int* __restrict__ err) {
-  constexpr int NB = 2 * N;  // GEMM columns: real parts, then imaginary parts
-  constexpr int NH = NB / 4;  // accumulator columns per thread (four warps per TMEM lane quarter)
+    far_tc_kernel(const __grid_constant__ Geometry g, const __grid_constant__ TcConst c,
+                  const float* __restrict__ ops, int64_t ntile_all, int nd,
+                  double* __restrict__ partial, int64_t chunk_len, int* __restrict__ err) {
+  constexpr int NB = 2 * N;               // accumulator columns: real, then imaginary parts
+  constexpr int NH = NB * 4 / kTcWarps;   // of which each thread sums
+  constexpr int SPLIT = kTcSplit<N>;
+  static_assert(SPLIT * 2 * NB + kTcACols <= int(kTcTmemCols), "tensor memory");
+  constexpr bool kTwoSums = N < 64;       // a second set of sums (64 densities: no registers left)
   constexpr uint32_t kLboB = (NB / 8) * 128;
-  constexpr uint32_t kCols = NB < 32 ? 32 : NB;  // tensor-memory allocation (power of 2 >= 32)
+  constexpr uint32_t kOpBytes = kTcOpFloats<N> * sizeof(float);
   extern __shared__ __align__(1024) unsigned char tc_smem[];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tmem_base;
-  __shared__ float4 sg0[kTcS];
-  __shared__ float2 sg1[kTcS];
-  __shared__ float4 sab[kTcS];
+  TcSmem<N>& sm = *reinterpret_cast<TcSmem<N>*>(
+      tc_smem + ((1024 - (smem_u32(tc_smem) & 1023)) & 1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  unsigned char* base = tc_smem + ((1024 - (smem_u32(tc_smem) & 1023)) & 1023);
-  float* sAh = reinterpret_cast<float*>(base);
-  float* sAl = sAh + kTcRows * kTcK;
-  float* sBh = sAl + kTcRows * kTcK;
-  float* sBl = sBh + NB * kTcK;
-
   const int64_t ntarg = g.ntarg, nptso = g.nptso;
   const int64_t tbase = int64_t(blockIdx.x) * kTcT;
   const int m0 = int(blockIdx.z) * N;
@@ -157,183 +286,332 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const int64_t tcen = (tbase / kFarBlockTargets32) * kFarBlockTargets32;
   const int64_t tcc = tcen < ntarg ? tcen : ntarg - 1;
   const double cx = g.tx[tcc], cy = g.ty[tcc], cz = g.tz[tcc];
-  // kernel values: target t against sources 4 (4 j + sgrp) .. + 3, j = 0, 1
-  const int t = tid & (kTcT - 1), sgrp = tid >> 7;
-  const int64_t it = tbase + t;
-  const int64_t ic = it < ntarg ? it : ntarg - 1;
-  const float tx = float(g.tx[ic] - cx), ty = float(g.ty[ic] - cy), tz = float(g.tz[ic] - cz);
-  const float thr2 = float(kp.thresh * kp.thresh);
-  const float k = float(kp.kr), kim = float(kp.ki);
-  // accumulator: row (target) 32 (warp % 4) + lane, columns c0 .. c0 + NH - 1
-  const int row = 32 * (warp & 3) + lane, c0 = (warp >> 2) * NH;
+  const int64_t s0 = int64_t(blockIdx.y) * chunk_len;
+  const int64_t s1 = s0 + chunk_len < nptso ? s0 + chunk_len : nptso;
+  const int ntiles = s1 > s0 ? int((s1 - s0 + kTcS - 1) / kTcS) : 0;
 
-  if (warp == 0) {
+  if (warp == kTcWarps + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(&tmem_base)),
-                 "r"(kCols));
+                     smem_u32(&sm.tmem)),
+                 "r"(kTcTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)));
+    auto init = [](uint64_t* b, int n) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n));
+    };
+    for (int s = 0; s < kTcStages; ++s) {
+      init(&sm.full[s], 1);
+      init(&sm.empty[s], kTcWarps + 1);
+    }
+    init(&sm.afull, kTcWarps);
+    init(&sm.done, 1);
+    sm.fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_base;
-  // operand descriptors of the three products hi*hi, hi*lo, lo*hi
-  const uint64_t desc_a[3] = {smem_desc(smem_u32(sAh), kTcLboA), smem_desc(smem_u32(sAh), kTcLboA),
-                              smem_desc(smem_u32(sAl), kTcLboA)};
-  const uint64_t desc_b[3] = {smem_desc(smem_u32(sBh), kLboB), smem_desc(smem_u32(sBl), kLboB),
-                              smem_desc(smem_u32(sBh), kLboB)};
+  const uint32_t tmem = sm.tmem;
+  const uint32_t acol = tmem + SPLIT * 2 * NB;  // A behind the accumulators
+  volatile int* fail = &sm.fail;
 
-  float acc[NH], cmp[NH];
+  if (warp < kTcWarps) {
+    const int quarter = warp & 3, sgrp = warp >> 2;
+    const uint32_t lanes = uint32_t(quarter * 32) << 16;
+    const int64_t to = tbase + 32 * quarter + lane;
+    const int64_t ic = to < ntarg ? to : ntarg - 1;
+    const float fx = float(g.tx[ic] - cx), fy = float(g.ty[ic] - cy), fz = float(g.tz[ic] - cz);
+    const float2 tx = make_float2(fx, fx), ty = make_float2(fy, fy), tz = make_float2(fz, fz);
+    const int c0 = sgrp * NH;  // this thread's accumulator columns
+    float2 sum[NH / 2];
+    double sum2[kTwoSums ? NH : 1];
 #pragma unroll
-  for (int n = 0; n < NH; ++n) acc[n] = cmp[n] = 0.f;
-  const int64_t s0 = int64_t(blockIdx.y) * chunk_len;
-  const int64_t s1 = s0 + chunk_len < nptso ? s0 + chunk_len : nptso;
-  const int ntiles = s1 > s0 ? int((s1 - s0 + kTcS - 1) / kTcS) : 0;
-  auto tile_ns = [&](int i) {
-    const int64_t sb = s0 + int64_t(i) * kTcS;
-    return int(s1 - sb < kTcS ? s1 - sb : kTcS);
-  };
-  TileRegs<N> pre;
-  if (ntiles > 0) tile_load<N>(g, ab, sig, nd, m0, s0, tile_ns(0), pre);
-  bool ok = true;
-  int issued = -1;  // last tile whose MMAs were committed
-  for (int i = 0; i < ntiles; ++i) {
-    const int ns = tile_ns(i);
-    if (i > 0) {
-      // tile i-1's MMAs read the operand buffers and wrote the accumulator
-      ok = wait_phase(&bar, uint32_t(i - 1) & 1u);
-      if (!ok) break;
+    for (int n = 0; n < NH / 2; ++n) sum[n] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int n = 0; n < NH; ++n) sum2[kTwoSums ? n : 0] = 0.0;
+    bool ok = true;
+    auto drain = [&](int i) {  // tile i's accumulator into the registers
+      ok = tc_wait_warp(&sm.done, uint32_t(i) & 1u, fail);
+      if (!ok) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      flush<NH>(tmem, c0, acc, cmp);
-    }
-    // the prefetched tile -> shared memory
-    if (tid < kTcS) {
-      if (tid < ns) {
-        sg0[tid] = make_float4(float(pre.sx - cx), float(pre.sy - cy), float(pre.sz - cz),
-                               float(pre.nx));
-        sg1[tid] = make_float2(float(pre.ny), float(pre.nz));
-        sab[tid] = pre.abv;
-      } else {
-        sg0[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
-        sg1[tid] = make_float2(0.f, 0.f);
-        sab[tid] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-    // densities: column n (real part of density m0 + n) = [sr; -si], column
-    // N + n (imaginary part) = [si; sr], over sources s (rows s, 32 + s)
+      flush_add<N, NH, SPLIT>(tmem + lanes, c0, sum);
+      if (kTwoSums && i % kTcFold == kTcFold - 1) {
 #pragma unroll
-    for (int kq = 0; kq < TileRegs<N>::kTasks; ++kq) {
-      const int q = tid + kq * kTcThreads;
-      if (q < N * (kTcS / 4)) {
-        const int n = q % N, sq = 4 * (q / N);
-        const float2* v = pre.sig[kq];
-        store_split(sBh, sBl, op_off(n, sq, kLboB), v[0].x, v[1].x, v[2].x, v[3].x);
-        store_split(sBh, sBl, op_off(n, kTcS + sq, kLboB), -v[0].y, -v[1].y, -v[2].y, -v[3].y);
-        store_split(sBh, sBl, op_off(N + n, sq, kLboB), v[0].y, v[1].y, v[2].y, v[3].y);
-        store_split(sBh, sBl, op_off(N + n, kTcS + sq, kLboB), v[0].x, v[1].x, v[2].x, v[3].x);
-      }
-    }
-    __syncthreads();
-    // kernel values of the tile: [Kr | Ki] for this thread's target
-#pragma unroll 1
-    for (int j = 0; j < kTcS / 16; ++j) {
-      const int sq = 4 * (4 * j + sgrp);
-      float kr[4], ki[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        kr[u] = 0.f;
-        ki[u] = 0.f;
-        pair_helm(tx, ty, tz, sg0[sq + u], sg1[sq + u], sab[sq + u], k, kim, thr2, CK, kr[u],
-                  ki[u]);
-      }
-      store_split(sAh, sAl, op_off(t, sq, kTcLboA), kr[0], kr[1], kr[2], kr[3]);
-      store_split(sAh, sAl, op_off(t, kTcS + sq, kTcLboA), ki[0], ki[1], ki[2], ki[3]);
-    }
-    // make the operands visible to the tensor core, then one thread issues
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (tid == 0) {
-      constexpr uint32_t idesc = idesc_tf32(kTcRows, NB);
-      uint32_t accf = 0u;
-#pragma unroll
-      for (int p = 0; p < 3; ++p)
-#pragma unroll
-        for (int st = 0; st < kTcK / 8; ++st) {
-          // K step st: two K-direction core matrices further
-          const uint64_t da = desc_a[p] + uint64_t(st * ((2 * kTcLboA) >> 4));
-          const uint64_t db = desc_b[p] + uint64_t(st * ((2 * kLboB) >> 4));
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::
-                  "r"(tmem),
-              "l"(da), "l"(db), "r"(idesc), "r"(accf), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-          accf = 1u;
+        for (int n = 0; n < NH / 2; ++n) {
+          sum2[kTwoSums ? 2 * n : 0] += double(sum[n].x);
+          sum2[kTwoSums ? 2 * n + 1 : 0] += double(sum[n].y);
+          sum[n] = make_float2(0.f, 0.f);
         }
-      asm volatile(
-          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-              smem_u32(&bar))
-          : "memory");
+      }
+    };
+    const uint32_t a0 = acol + lanes + uint32_t(kTcPer * sgrp);
+    for (int i = 0; i < ntiles; ++i) {
+      const int s = i % kTcStages;
+      ok = tc_wait_warp(&sm.full[s], uint32_t(i / kTcStages) & 1u, fail);
+      if (!ok) break;
+      const TcGeom& ge = sm.geom[s];
+      float vr[kTcPer], vi[kTcPer];
+      auto eval = [&](auto chk) {
+        constexpr bool C = decltype(chk)::value;
+#pragma unroll
+        for (int j = 0; j < kTcPer; j += 4) {
+          const int q = kTcPer * sgrp + j;
+          const float4 x = *reinterpret_cast<const float4*>(ge.x + q);
+          const float4 y = *reinterpret_cast<const float4*>(ge.y + q);
+          const float4 z = *reinterpret_cast<const float4*>(ge.z + q);
+          const float4 nx = *reinterpret_cast<const float4*>(ge.nx + q);
+          const float4 ny = *reinterpret_cast<const float4*>(ge.ny + q);
+          const float4 nz = *reinterpret_cast<const float4*>(ge.nz + q);
+          float2 a, b;
+          tc_pair<C, CK>(tx, ty, tz, make_float2(x.x, x.y), make_float2(y.x, y.y),
+                         make_float2(z.x, z.y), make_float2(nx.x, nx.y), make_float2(ny.x, ny.y),
+                         make_float2(nz.x, nz.y), c, a, b);
+          vr[j] = a.x, vr[j + 1] = a.y, vi[j] = b.x, vi[j + 1] = b.y;
+          tc_pair<C, CK>(tx, ty, tz, make_float2(x.z, x.w), make_float2(y.z, y.w),
+                         make_float2(z.z, z.w), make_float2(nx.z, nx.w), make_float2(ny.z, ny.w),
+                         make_float2(nz.z, nz.w), c, a, b);
+          vr[j + 2] = a.x, vr[j + 3] = a.y, vi[j + 2] = b.x, vi[j + 3] = b.y;
+        }
+      };
+      if (ge.check)
+        eval(std::true_type{});
+      else
+        eval(std::false_type{});
+      __syncwarp();
+      if (lane == 0) tc_arrive(&sm.empty[s]);
+      // the tensor core is done with the previous tile's A and accumulators
+      if (i > 0) {
+        drain(i - 1);
+        if (!ok) break;
+      }
+      split_store16(a0, a0 + 2 * kTcS, vr);
+      split_store16(a0 + kTcS, a0 + 3 * kTcS, vi);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc_arrive(&sm.afull);
     }
-    issued = i;
-    // the next tile's operands load while the tensor core works
-    if (i + 1 < ntiles) tile_load<N>(g, ab, sig, nd, m0, s0 + int64_t(i + 1) * kTcS, tile_ns(i + 1), pre);
-  }
-  if (ok && ntiles > 0) {
-    ok = wait_phase(&bar, uint32_t(ntiles - 1) & 1u);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) flush<NH>(tmem, c0, acc, cmp);
-  }
-  if (!ok) {
-    if (tid == 0 && err) atomicExch(err, 1 + int(blockIdx.x));
-    // let the last committed MMAs finish before the tensor memory is freed
-    for (uint32_t r = 0; r < 4 && issued >= 0; ++r)
-      if (wait_phase(&bar, uint32_t(issued) & 1u)) break;
-  } else {
-    // row: target tbase + row; column c0 + n: real (< N) or imaginary part of
-    // density m0 + (c0 + n) % N
-    const int64_t to = tbase + row;
-    const int comp = c0 >= N ? 1 : 0, d0 = m0 + (c0 % N);
-    if (to < ntarg)
+    if (ok && ntiles > 0) drain(ntiles - 1);
+    if (ok && to < ntarg) {
+      // column c0 + n: real (< N) or imaginary part of density m0 + (c0 + n) % N
+      const int comp = c0 >= N ? 1 : 0, d0 = m0 + (c0 % N);
 #pragma unroll
       for (int n = 0; n < NH; ++n)
-        if (d0 + n < nd)
+        if (d0 + n < nd) {
+          const double v = double(n & 1 ? sum[n / 2].y : sum[n / 2].x);
           partial[((size_t(blockIdx.y) * ntarg + to) * nd + d0 + n) * 2 + comp] =
-              double(acc[n]) - double(cmp[n]);
+              kTwoSums ? sum2[kTwoSums ? n : 0] + v : v;
+        }
+    }
+  } else if (warp == kTcWarps) {
+    // producer: lane j takes sources j, 32 + j of each tile.  The coordinates and the
+    // bounding box of the next tile load while this one goes out.
+    constexpr int H = kTcS / 32;
+    const float* op = ops + (size_t(blockIdx.z) * ntile_all + size_t(s0 / kTcS)) * kTcOpFloats<N>;
+    const double* tb = g.tbox && g.sbox ? g.tbox + 6 * (tbase / kFarBlockTargets32) : nullptr;
+    double raw[H][6], sbx = 0.0;
+    // lane d < 3: the target box's range in dimension d
+    const double tlo = tb && lane < 3 ? tb[lane] : 0.0, thi = tb && lane < 3 ? tb[lane + 3] : 0.0;
+    auto fetch = [&](int64_t sg) {  // the tile of sources from sg on
+#pragma unroll
+      for (int u = 0; u < H; ++u) {
+        const int64_t s = sg + u * 32 + lane;
+        const bool in = s < s1;
+        // a padding source sits at the block centre: it keeps the threshold
+        // test of its tile and meets zero densities
+        raw[u][0] = in ? g.sx[s] : cx;
+        raw[u][1] = in ? g.sy[s] : cy;
+        raw[u][2] = in ? g.sz[s] : cz;
+        raw[u][3] = in ? g.snx[s] : 0.0;
+        raw[u][4] = in ? g.sny[s] : 0.0;
+        raw[u][5] = in ? g.snz[s] : 0.0;
+      }
+      if (tb && lane < 6 && sg < s1) sbx = g.sbox[6 * (sg / kFarTileSources) + lane];
+    };
+    if (ntiles > 0) fetch(s0);
+    int issued = 0;
+    for (int i = 0; i < ntiles; ++i) {
+      const int s = i % kTcStages;
+      const int64_t sg = s0 + int64_t(i) * kTcS;
+      float cur[H][6];
+#pragma unroll
+      for (int u = 0; u < H; ++u) {
+        cur[u][0] = -float(raw[u][0] - cx);
+        cur[u][1] = -float(raw[u][1] - cy);
+        cur[u][2] = -float(raw[u][2] - cz);
+#pragma unroll
+        for (int d = 3; d < 6; ++d) cur[u][d] = float(raw[u][d]);
+      }
+      const double shi = __shfl_down_sync(0xffffffffu, sbx, 3);
+      const double gap = lane < 3 ? fmax(fmax(sbx - thi, tlo - shi), 0.0) : 0.0;
+      const double g2 = gap * gap;
+      const double gap2 = g2 + __shfl_down_sync(0xffffffffu, g2, 1) + __shfl_down_sync(0xffffffffu, g2, 2);
+      if (i + 1 < ntiles) fetch(sg + kTcS);
+      if (i >= kTcStages && !tc_wait_warp(&sm.empty[s], uint32_t(i / kTcStages - 1) & 1u, fail)) break;
+      TcGeom& ge = sm.geom[s];
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+        const int j = 32 * h + lane;
+        ge.x[j] = cur[h][0];
+        ge.y[j] = cur[h][1];
+        ge.z[j] = cur[h][2];
+        ge.nx[j] = cur[h][3];
+        ge.ny[j] = cur[h][4];
+        ge.nz[j] = cur[h][5];
+      }
+      // only a whole tile may skip the threshold test (padding needs it)
+      if (lane == 0) ge.check = !tb || sg + kTcS > s1 || gap2 <= g.box_margin2;
+      __syncwarp();
+      if (lane == 0) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                         smem_u32(&sm.full[s])),
+                     "r"(kOpBytes)
+                     : "memory");
+        asm volatile(
+            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+            "[%3];" ::"r"(smem_u32(sm.b[s])),
+            "l"(op + size_t(i) * kTcOpFloats<N>), "r"(kOpBytes), "r"(smem_u32(&sm.full[s]))
+            : "memory");
+      }
+      issued = i + 1;
+    }
+    if (*fail)  // the copies still in flight land before the CTA goes
+      for (int i = issued > kTcStages ? issued - kTcStages : 0; i < issued; ++i)
+        for (uint32_t r = 0; r < kTcSpin; ++r) {
+          uint32_t done;
+          asm volatile(
+              "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+              "selp.b32 %0, 1, 0, p;\n\t}\n"
+              : "=r"(done)
+              : "r"(smem_u32(&sm.full[i % kTcStages])), "r"(uint32_t(i / kTcStages) & 1u)
+              : "memory");
+          if (done) break;
+        }
+  } else {
+    // the whole warp walks the tiles, so that the operands of the MMAs stay
+    // in uniform registers; one elected lane issues
+    constexpr uint32_t kAll = idesc_tf32(kTcT, NB);
+    const uint64_t bdesc = smem_desc(smem_u32(sm.b[0]), kLboB);
+    int issued = -1;
+    for (int i = 0; i < ntiles; ++i) {
+      const int s = i % kTcStages;
+      if (!tc_wait_warp(&sm.full[s], uint32_t(i / kTcStages) & 1u, fail)) break;
+      if (!tc_wait_warp(&sm.afull, uint32_t(i) & 1u, fail)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t bd = bdesc + uint64_t(uint32_t(s) * (kOpBytes >> 4));
+      if (elect_one()) {
+        // lo*hi, hi*lo, hi*hi
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+          const uint32_t ap = acol + (p == 0 ? 2 * kTcS : 0);
+          const uint64_t bp = bd + (p == 1 ? uint64_t(kOpBytes / 2) >> 4 : 0);
+#pragma unroll
+          for (int ks = 0; ks < kTcS / 8; ++ks) {
+            const uint64_t bk = bp + uint64_t((ks * 2 * kLboB) >> 4);
+            constexpr int per = kTcS / 8 / SPLIT;
+            const uint32_t d = tmem + uint32_t(ks / per) * 2 * NB;
+            if (p == 0 && ks % per == 0) {
+              tc_mma<false>(d, ap + 8 * ks, bk, kAll);
+              tc_mma<false>(d + NB, ap + kTcS + 8 * ks, bk, kAll);
+            } else {
+              tc_mma<true>(d, ap + 8 * ks, bk, kAll);
+              tc_mma<true>(d + NB, ap + kTcS + 8 * ks, bk, kAll);
+            }
+          }
+        }
+        tc_commit(&sm.done);
+        tc_commit(&sm.empty[s]);
+      }
+      __syncwarp();
+      issued = i;
+    }
+    if (*fail && issued >= 0) {
+      // let the last committed MMAs finish before the tensor memory is freed
+      for (uint32_t r = 0; r < kTcSpin; ++r) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(smem_u32(&sm.done)), "r"(uint32_t(issued) & 1u)
+            : "memory");
+        if (done) break;
+      }
+    }
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+  if (tid == 0 && *fail && err) atomicExch(err, 1 + int(blockIdx.x));
+  if (warp == kTcWarps + 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kTcTmemCols));
 }
 
+// B operand of every tile: the oversampled densities times weight / 4 pi,
+// split into high and low parts, rows real then imaginary, zero beyond the
+// last source and density.  One block per (tile, density group).
 template <int N>
-size_t tc_smem_bytes() {
-  return sizeof(float) * (2 * kTcRows * kTcK + 2 * (2 * N) * kTcK) + 1024;
+__global__ void far_tc_operand_kernel(Geometry g, const float* __restrict__ sig, int nd,
+                                      float* __restrict__ ops) {
+  constexpr uint32_t kLboB = (2 * N / 8) * 128;
+  const int64_t tile = blockIdx.x, sb = tile * kTcS;
+  const int m0 = int(blockIdx.y) * N;
+  __shared__ float sv[kTcS][2 * N + 1];
+  for (int q = threadIdx.x; q < kTcS * N; q += blockDim.x) {
+    const int j = q / N, m = q - j * N;
+    const int64_t s = sb + j;
+    float2 v = make_float2(0.f, 0.f);
+    if (s < g.nptso && m0 + m < nd) {
+      const double f = g.sw[s] * kTcOver4Pi;
+      const float2 u = reinterpret_cast<const float2*>(sig)[size_t(s) * nd + m0 + m];
+      v = make_float2(float(double(u.x) * f), float(double(u.y) * f));
+    }
+    sv[j][m] = v.x;
+    sv[j][N + m] = v.y;
+  }
+  __syncthreads();
+  float* hi = ops + (size_t(blockIdx.y) * gridDim.x + tile) * kTcOpFloats<N>;
+  float* lo = hi + kTcOpFloats<N> / 2;
+  for (int q = threadIdx.x; q < 2 * N * (kTcS / 4); q += blockDim.x) {
+    const int r = q % (2 * N), k = 4 * (q / (2 * N));
+    store_split(hi, lo, op_off(r, k, kLboB), sv[k][r], sv[k + 1][r], sv[k + 2][r], sv[k + 3][r]);
+  }
 }
 
 template <int N, bool CK>
 cudaError_t far_tc_go(const Geometry& g, const KParams& kp, const MatvecArgs& a, cudaStream_t st,
                       int* occ) {
   auto kern = far_tc_kernel<N, CK>;
-  const size_t smem = tc_smem_bytes<N>();
+  const size_t smem = sizeof(TcSmem<N>) + 1024;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(smem));
   if (e != cudaSuccess) return e;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, kTcThreads, smem);
+  if (!a.tc_ops) return cudaErrorInvalidValue;
   const int64_t tblocks = (g.ntarg + kTcT - 1) / kTcT;
   const int groups = (a.nd + N - 1) / N;
+  const int64_t ntile = (g.nptso + kTcS - 1) / kTcS;
   int64_t chunk = (g.nptso + a.nchunks - 1) / a.nchunks;
   chunk = ((chunk + kFarTileSources - 1) / kFarTileSources) * kFarTileSources;
+  far_tc_operand_kernel<N><<<dim3(unsigned(ntile), unsigned(groups)), 256, 0, st>>>(
+      g, static_cast<const float*>(a.strengths), a.nd, a.tc_ops);
+  note_launches(1);
   const dim3 grid(unsigned(tblocks), unsigned(a.nchunks), unsigned(groups));
-  kern<<<grid, kTcThreads, smem, st>>>(g, kp, static_cast<const float*>(a.ab),
-                                       static_cast<const float*>(a.strengths), a.nd, a.partial,
-                                       chunk, a.tc_err);
+  auto dup = [](double v) { return make_float2(float(v), float(v)); };
+  TcConst c;
+  c.k = dup(kp.kr);
+  c.kim = dup(kp.ki);
+  c.ar = dup(kp.ar);
+  c.ai = dup(kp.ai);
+  c.br = dup(kp.br);
+  c.bi = dup(kp.bi);
+  c.mbr = dup(-kp.br);
+  c.one = dup(1.0);
+  c.mone = dup(-1.0);
+  c.thr2 = float(kp.thresh * kp.thresh);
+  kern<<<grid, kTcThreads, smem, st>>>(g, c, a.tc_ops, ntile, a.nd, a.partial, chunk, a.tc_err);
   return cudaGetLastError();
 }
 
@@ -349,9 +627,18 @@ cudaError_t far_tc_n(const Geometry& g, const KParams& kp, const MatvecArgs& a, 
 int far_tc_targets() { return kTcT; }
 
 int far_tc_group(int variant, int nd, int precision, int kind) {
-  if (variant < 3 || variant > 4 || precision != 1 || kind != 1 || nd < 4) return 0;
+  if (variant < 3 || variant > 4 || precision != 1 || kind != 1 || nd < 2) return 0;
   if (variant == 4) return nd > 32 ? 64 : 0;
   return nd <= 16 ? 16 : 32;
+}
+
+size_t far_tc_operand_floats(int nd, int precision, int kind, int64_t nptso) {
+  size_t most = 0;
+  for (int v = 3; v <= 4; ++v) {
+    const int n = far_tc_group(v, nd, precision, kind);
+    if (n > 0) most = std::max(most, size_t((nd + n - 1) / n) * n);
+  }
+  return most * size_t((nptso + kTcS - 1) / kTcS) * (2 * 2 * kTcS);
 }
 
 cudaError_t far_tc(int variant, const Geometry& g, const KParams& kp, const MatvecArgs& a,

@@ -716,10 +716,11 @@ cudaError_t Plan::launch_far_stage(const dev::MatvecArgs& a, cudaStream_t st) {
 }
 
 int Plan::ensure_workspace(int precision, int nd, int nchunks) {
-  (void)precision;
   const size_t sreals = size_t(nptso) * nd * (cplx ? 4 : 2);
   BIE_CUDA(str_.alloc(sreals * sizeof(double)));
   BIE_CUDA(partial_.alloc(std::max<size_t>(1, size_t(nchunks) * ntarg * nd * (cplx ? 2 : 1))));
+  if (far_method_[precision & 1] == 0)
+    BIE_CUDA(tc_ops_.alloc(dev::far_tc_operand_floats(nd, precision, kind, nptso)));
   return kOk;
 }
 
@@ -819,6 +820,7 @@ int Plan::matvec(int precision, int nd, const double* d_sigma, double* d_pot, cu
   a.weff_f32 = precision == 1;
   a.ab = precision == 1 ? (const void*)ab32_.p : (const void*)ab64_.p;
   a.tc_err = tc_err_.p;
+  a.tc_ops = tc_ops_.p;
   if (timing) BIE_CUDA(cudaEventRecord(ev_[0], st));
   if (nd > 1)
     BIE_CUDA(oversample(a, st));

@@ -271,6 +271,7 @@ class Plan : public Operator {
   DBuf<int64_t> cmoff_, row_ptr_, wofs_;
   DBuf<double> weff64_;
   DBuf<float> weff32_;
+  DBuf<float> tc_ops_;  // its density operand
   DBuf<int> tc_err_;  // timeout flag of the tensor-core far field
   std::unique_ptr<TreeFar> tree_[2];
   int far_method_[2] = {0, 0};

@@ -380,7 +380,7 @@ int bie_plan_oversample(void* plan, int64_t engine, int64_t nd, const double* si
                         float* out_dev, void* stream);
 /* Far-field shape of (iprec, nd): bie_plan_set_far pins it (variant 0-2:
  * CUDA-core block shapes; 3-4: tensor-core kernel of the FP32 Helmholtz
- * multi-density path, 16/32 or 64 densities per CTA, nd >= 4; nchunks source
+ * multi-density path, 16/32 or 64 densities per CTA, nd >= 2; nchunks source
  * chunks) instead of the autotuner's choice; bie_plan_get_far returns the
  * variant, the chunk count and a nonzero flag if a tensor-core launch timed
  * out waiting for its MMAs.  No reference counterpart. */
