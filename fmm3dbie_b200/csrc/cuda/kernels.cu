@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(NT, (kFarMinBlocks<R, NT>)) far_kernel(Geometr
     __shared__ double2 stab[KIND == 1 ? kFarTrigN : 1];
     const double2* tab = nullptr;
     if constexpr (KIND == 1) {
-      fill_far_trig_table(stab);  // published by the first __syncthreads of the tile loop
+      fill_far_trig_table(stab);
       tab = stab;
     }
     far_block<KIND, R, NT, TPT, TILE, CK>(g, kp, str, partial, chunk_len, nd, blockIdx.x,
@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(NT) far_md_kernel(Geometry g, KParams kp,
   __shared__ double2 stab[sizeof(R) == 8 && KIND == 1 ? kFarTrigN : 1];
   const double2* tab = nullptr;
   if constexpr (sizeof(R) == 8 && KIND == 1) {
-    fill_far_trig_table(stab);  // published by the first __syncthreads of the tile loop
+    fill_far_trig_table(stab);
     tab = stab;
   }
   far_md_block<KIND, R, NT, TPT, MD, TILE, CK>(g, kp, ab, sig, nd, partial, chunk_len, blockIdx.x,
@@ -1646,6 +1646,11 @@ constexpr int kMdShapes[3][3][3] = {
     {{128, 1, 8}, {128, 2, 8}, {64, 2, 8}},
     {{128, 1, 16}, {64, 1, 16}, {256, 1, 16}}};
 
+// Sources per tile: FP64 blocks of 16 densities take half tiles, so that the
+// densities and the sine/cosine table fit the static shared memory.
+template <typename R, int MD>
+constexpr int kMdTile = sizeof(R) == 8 && MD == 16 ? kFarTile / 2 : kFarTile;
+
 inline int md_class(int nd) { return nd <= 4 ? 0 : (nd <= 8 ? 1 : 2); }
 
 template <int KIND, typename R, bool CK, int CL, int V>
@@ -1654,7 +1659,7 @@ cudaError_t far_md_dispatch(const Geometry& g, const KParams& kp, const MatvecAr
   constexpr int NT = kMdShapes[CL][V][0], TPT = kMdShapes[CL][V][1], MD = kMdShapes[CL][V][2];
   if (occ) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        occ, far_md_kernel<KIND, R, NT, TPT, MD, kFarTile, CK>, NT, 0);
+        occ, far_md_kernel<KIND, R, NT, TPT, MD, kMdTile<R, MD>, CK>, NT, 0);
     return cudaSuccess;
   }
   const int64_t tblocks = (g.ntarg + int64_t(NT) * TPT - 1) / (int64_t(NT) * TPT);
@@ -1663,7 +1668,7 @@ cudaError_t far_md_dispatch(const Geometry& g, const KParams& kp, const MatvecAr
   chunk = ((chunk + kFarTile - 1) / kFarTile) * kFarTile;
   const dim3 grid(static_cast<unsigned>(tblocks), static_cast<unsigned>(a.nchunks),
                   static_cast<unsigned>(groups));
-  far_md_kernel<KIND, R, NT, TPT, MD, kFarTile, CK><<<grid, NT, 0, st>>>(
+  far_md_kernel<KIND, R, NT, TPT, MD, kMdTile<R, MD>, CK><<<grid, NT, 0, st>>>(
       g, kp, static_cast<const R*>(a.ab), static_cast<const R*>(a.strengths), a.nd, a.partial,
       chunk);
   return cudaGetLastError();
@@ -1894,7 +1899,7 @@ cudaError_t batch_far_dispatch(const BatchArgs& a, cudaStream_t st, int* occ) {
 template <int KIND, typename R, bool CK, int CL, int V>
 cudaError_t batch_far_md_dispatch(const BatchArgs& a, cudaStream_t st, int* occ) {
   constexpr int NT = kMdShapes[CL][V][0], TPT = kMdShapes[CL][V][1], MD = kMdShapes[CL][V][2];
-  auto kern = batch_far_md_kernel<KIND, R, NT, TPT, MD, kFarTile, CK>;
+  auto kern = batch_far_md_kernel<KIND, R, NT, TPT, MD, kMdTile<R, MD>, CK>;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, NT, 0);
   kern<<<a.grid_far, NT, 0, st>>>(a.surfs, a.far_items, a.nfar_items,
                                   static_cast<const R*>(a.str), a.partial, a.nd, a.precision,

@@ -133,24 +133,38 @@ __device__ __forceinline__ void lagrange_d(int p, R u, R* L, R* D) {
 constexpr int kUpThreads = 128, kUpTile = 32;
 constexpr int64_t kUpChunk = 2048;
 
+// Groups along the third side of a pxy x pz grid (one thread per (i, j) and
+// group; at most 8 points a group, for the registers) and points per group.
+__device__ __forceinline__ int up_groups(int pxy, int pz) {
+  return min(max(kUpThreads / pxy, (pz + 7) / 8), pz);
+}
+
 // SIG = false: str holds each source's (charge, dipole) strengths per
 // density; SIG = true: they are formed as (a_s sigma_m, b_s sigma_m) from
-// the oversampled densities sig and the per-source constants ab.
-template <int KIND, typename R, bool SIG>
-__global__ void __launch_bounds__(kUpThreads)
-    tree_up_kernel(const UpItemD* __restrict__ items, TreeArgs ta, const R* __restrict__ str,
-                   const R* __restrict__ sig, const R* __restrict__ ab, int nd,
-                   double* __restrict__ up_part) {
+// the oversampled densities sig and the per-source constants ab.  LC: grid
+// points along the third side per thread.
+template <typename R, int SW>
+struct UpSmem {
+  R L[3][kP + 2][kUpTile];  // two spare rows: the last group of LC rows may run past kP
+  R D[3][kP + 2][kUpTile];  // derivative along the side times the normal component
+  R S[kUpTile][SW];
+};
+
+template <int KIND, typename R, bool SIG, int LC>
+__device__ __forceinline__ void tree_up_body(const UpItemD& it, const TreeArgs& ta,
+                                             const R* __restrict__ str, const R* __restrict__ sig,
+                                             const R* __restrict__ ab, int nd,
+                                             double* __restrict__ up_part,
+                                             UpSmem<R, KIND == 1 ? 4 : 2>& sm) {
   constexpr int SW = KIND == 1 ? 4 : 2;
   constexpr int C = KIND == 1 ? 2 : 1;
-  __shared__ R sL[3][kP][kUpTile];
-  __shared__ R sD[3][kP][kUpTile];  // derivative along the side times the normal component
-  __shared__ R sS[kUpTile][SW];
-  const UpItemD it = items[blockIdx.x];
+  auto& sL = sm.L;
+  auto& sD = sm.D;
+  auto& sS = sm.S;
   const int m = blockIdx.y, tid = threadIdx.x;
   const int npd[3] = {it.np0, it.np1, it.np2};
   const int pxy = it.np0 * it.np1, pz = it.np2;
-  const int lg = min(max(kUpThreads / pxy, 1), pz);  // l-groups per (i, j)
+  const int lg = up_groups(pxy, pz);                 // l-groups per (i, j)
   const int lc = (pz + lg - 1) / lg;                 // l per group
   const int slots = pxy * lg;
   double ctr[3], h[3];
@@ -166,9 +180,9 @@ __global__ void __launch_bounds__(kUpThreads)
     const int i = ij / it.np1, j = ij - (ij / it.np1) * it.np1;
     const int l0 = grp * lc;
     const int nl = act ? max(0, min(lc, pz - l0)) : 0;
-    double accr[kP], acci[kP];
+    double accr[LC], acci[LC];
 #pragma unroll
-    for (int l = 0; l < kP; ++l) accr[l] = acci[l] = 0.0;
+    for (int l = 0; l < LC; ++l) accr[l] = acci[l] = 0.0;
     for (int64_t sb = it.b; sb < it.e; sb += kUpTile) {
       const int ns = int(it.e - sb < kUpTile ? it.e - sb : kUpTile);
       __syncthreads();
@@ -212,9 +226,10 @@ __global__ void __launch_bounds__(kUpThreads)
       }
       __syncthreads();
       if (nl > 0) {
-        R tr[kP], ti[kP];
+        R tr[LC], ti[LC];
 #pragma unroll
-        for (int l = 0; l < kP; ++l) tr[l] = ti[l] = R(0);
+        for (int l = 0; l < LC; ++l) tr[l] = ti[l] = R(0);
+#pragma unroll 2
         for (int s = 0; s < ns; ++s) {
           const R lx = sL[0][i][s], dx = sD[0][i][s], ly = sL[1][j][s], dy = sD[1][j][s];
           const R v = lx * ly, gxy = fma(dx, ly, lx * dy);
@@ -228,29 +243,50 @@ __global__ void __launch_bounds__(kUpThreads)
             ar = fma(sS[s][0], v, sS[s][1] * gxy);
             br = sS[s][1] * v;
           }
+          // a group's last l may lie beyond pz: its sums are not written
 #pragma unroll
-          for (int l = 0; l < kP; ++l)
-            if (l < nl) {
-              const R lz = sL[2][l0 + l][s], dz = sD[2][l0 + l][s];
-              tr[l] = fma(ar, lz, fma(br, dz, tr[l]));
-              if constexpr (KIND == 1) ti[l] = fma(ai, lz, fma(bi, dz, ti[l]));
-            }
+          for (int l = 0; l < LC; ++l) {
+            const R lz = sL[2][l0 + l][s], dz = sD[2][l0 + l][s];
+            tr[l] = fma(ar, lz, fma(br, dz, tr[l]));
+            if constexpr (KIND == 1) ti[l] = fma(ai, lz, fma(bi, dz, ti[l]));
+          }
         }
 #pragma unroll
-        for (int l = 0; l < kP; ++l) {
+        for (int l = 0; l < LC; ++l) {
           accr[l] += double(tr[l]);
           acci[l] += double(ti[l]);
         }
       }
     }
 #pragma unroll
-    for (int l = 0; l < kP; ++l)
+    for (int l = 0; l < LC; ++l)
       if (l < nl) {
         const int64_t k = int64_t(i * it.np1 + j) * pz + l0 + l;
         double* o = up_part + ((it.ubase + k) * nd + m) * C;
         o[0] = accr[l];
         if constexpr (C == 2) o[1] = acci[l];
       }
+  }
+}
+
+// The points per thread are a compile-time count: with a loop to kP guarded by
+// l < nl every source took the issue slots of 16 grid points.
+template <int KIND, typename R, bool SIG>
+__global__ void __launch_bounds__(kUpThreads)
+    tree_up_kernel(const UpItemD* __restrict__ items, TreeArgs ta, const R* __restrict__ str,
+                   const R* __restrict__ sig, const R* __restrict__ ab, int nd,
+                   double* __restrict__ up_part) {
+  __shared__ UpSmem<R, KIND == 1 ? 4 : 2> sm;
+  const UpItemD it = items[blockIdx.x];
+  const int lg = up_groups(it.np0 * it.np1, it.np2);
+  switch ((it.np2 + lg - 1) / lg) {
+    case 1: return tree_up_body<KIND, R, SIG, 1>(it, ta, str, sig, ab, nd, up_part, sm);
+    case 2: return tree_up_body<KIND, R, SIG, 2>(it, ta, str, sig, ab, nd, up_part, sm);
+    case 3: return tree_up_body<KIND, R, SIG, 3>(it, ta, str, sig, ab, nd, up_part, sm);
+    case 4: return tree_up_body<KIND, R, SIG, 4>(it, ta, str, sig, ab, nd, up_part, sm);
+    case 5:
+    case 6: return tree_up_body<KIND, R, SIG, 6>(it, ta, str, sig, ab, nd, up_part, sm);
+    default: return tree_up_body<KIND, R, SIG, 8>(it, ta, str, sig, ab, nd, up_part, sm);
   }
 }
 
@@ -271,25 +307,191 @@ __global__ void tree_reduce_kernel(const RedD* __restrict__ reds, const double* 
 // ---------------------------------------------------------------------------
 // list evaluation
 // ---------------------------------------------------------------------------
-constexpr int kEvThreads = 128, kEvTile = 128;
+constexpr int kEvThreads = 128;  // targets of a leaf or proxy item at most; threads of the md form
+// Threads (and sources per tile) of the one-density form.  A leaf holds 64 to
+// 128 targets (64 or 78 on a 146,016-node surface), so its 192 threads are
+// (warp of targets) x (part of the tile's sources): two target warps take
+// thirds of every tile, three take halves, and no warp idles; proxy items
+// fill 128 threads.
+template <bool PROXYT>
+constexpr int kEvBlock = PROXYT ? 128 : 192;
 
+// Blocks per SM the one-density form is compiled for (FP64 Helmholtz keeps up
+// to 168 registers: one block more measured 2 % slower; FP32 80: one block
+// fewer or more measured within 1 %).
+template <int KIND, typename R, bool PROXYT>
+constexpr int kEvMinBlocks = sizeof(R) == 4 ? (PROXYT ? 6 : 4)
+                             : KIND == 1    ? (PROXYT ? 3 : 2)
+                                            : (PROXYT ? 4 : 3);
+
+// The source tiles of a work item, in order: the entries of its node and,
+// for a leaf, of every ancestor.
+template <bool PROXYT, int TILE>
+struct TileIter {
+  const TNodeD* tn;
+  const EntryD* ents;
+  int64_t q, e1;
+  int n, sb;
+  EntryD en;
+  bool valid;
+  __device__ __forceinline__ void seek() {  // first entry at or after q
+    while (q >= e1) {
+      if (PROXYT || (n = tn[n].parent) < 0) {
+        valid = false;
+        return;
+      }
+      q = tn[n].pe0;
+      e1 = tn[n].pe1;
+    }
+    en = ents[q];
+    sb = en.b;
+  }
+  __device__ __forceinline__ void start(const TreeArgs& ta, int node, const TNodeD& t) {
+    tn = ta.tn;
+    ents = PROXYT ? ta.cent : ta.pent;
+    n = node;
+    q = PROXYT ? t.ce0 : t.pe0;
+    e1 = PROXYT ? t.ce1 : t.pe1;
+    valid = true;
+    seek();
+  }
+  __device__ __forceinline__ void next() {
+    sb += TILE;
+    if (sb >= en.e) {
+      ++q;
+      seek();
+    }
+  }
+};
+
+// One source of a tile as loaded (before centring and conversion): the next
+// tile's loads are in flight while the present one is evaluated.
+template <typename R>
+struct RawSource {
+  double x, y, z, nx, ny, nz;
+  typename Vec<R>::T4 s;
+};
+
+// A tile in shared memory.  FP32: one array per value, the coordinates
+// negated, so that a thread reads four consecutive sources at a time and
+// evaluates two per packed instruction; FP64: one record per source.
+template <int KIND, typename R, int TILE>
+struct TileSmem {
+  double4 g0[TILE];
+  double2 g1[TILE];
+  double4 st[TILE];
+};
+template <int KIND, int TILE>
+struct TileSmem<KIND, float, TILE> {
+  float v[KIND == 1 ? 10 : 8][TILE];  // x, y, z, nx, ny, nz, charge, dipole
+};
+
+// FP32: the tile's sources j0 .. j1 - 1 (a multiple of 4; sources past the
+// tile's end carry no strength) against one target, two per packed
+// instruction, two at a time; per lane the operations of pair_helm,
+// pair_lap and pair_charge.
+template <int KIND, bool CK, int MODE, int TILE>  // MODE: entry kind
+__device__ __forceinline__ void tile_eval(const TileSmem<KIND, float, TILE>& T, int j0, int j1,
+                                          float tx, float ty, float tz, float k, float kim,
+                                          float thr2, float& outr, float& outi) {
+  const float2 x = make_float2(tx, tx), y = make_float2(ty, ty), z = make_float2(tz, tz);
+  const float2 k2 = make_float2(k, k), kim2 = make_float2(kim, kim);
+  float2 pa = make_float2(0.f, 0.f), pb = pa, pi = pa;
+  auto at = [&](int a, int j) { return *reinterpret_cast<const float4*>(&T.v[a][j]); };
+  auto lo = [](const float4& q) { return make_float2(q.x, q.y); };
+  auto hi = [](const float4& q) { return make_float2(q.z, q.w); };
+  auto charge = [&](float2 sx, float2 sy, float2 sz, float2 cr, float2 ci) {
+    const float2 dx = __fadd2_rn(x, sx), dy = __fadd2_rn(y, sy), dz = __fadd2_rn(z, sz);
+    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+    float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+    if constexpr (KIND == 1) {
+      const float2 r = __fmul2_rn(r2, rinv), kr = __fmul2_rn(k2, r);
+      float2 sn, cs;
+      __sincosf(kr.x, &sn.x, &cs.x);
+      __sincosf(kr.y, &sn.y, &cs.y);
+      if (CK) {
+        rinv.x *= __expf(-kim * r.x);
+        rinv.y *= __expf(-kim * r.y);
+      }
+      const float2 er = __fmul2_rn(cr, rinv), ei = __fmul2_rn(ci, rinv);
+      pa = __ffma2_rn(cs, er, pa);
+      pb = __ffma2_rn(sn, ei, pb);
+      pi = __ffma2_rn(cs, ei, __ffma2_rn(sn, er, pi));
+    } else {
+      pa = __ffma2_rn(cr, rinv, pa);
+    }
+  };
+#pragma unroll 2
+  for (int j = j0; j < j1; j += 4) {
+    const float4 sx = at(0, j), sy = at(1, j), sz = at(2, j);
+    if constexpr (MODE == 2) {
+      const float4 cr = at(6, j), ci = KIND == 1 ? at(7, j) : cr;
+      charge(lo(sx), lo(sy), lo(sz), lo(cr), lo(ci));
+      charge(hi(sx), hi(sy), hi(sz), hi(cr), hi(ci));
+    } else {
+      const float4 nx = at(3, j), ny = at(4, j), nz = at(5, j);
+      if constexpr (KIND == 1) {
+        const float4 cr = at(6, j), ci = at(7, j), dr = at(8, j), di = at(9, j);
+        const float4 md = make_float4(-dr.x, -dr.y, -dr.z, -dr.w);
+        pair_helm_x2<MODE == 0>(x, y, z, lo(sx), lo(sy), lo(sz), lo(nx), lo(ny), lo(nz), lo(cr),
+                                lo(ci), lo(dr), lo(di), lo(md), k2, kim2, thr2, CK, pa, pb, pi);
+        pair_helm_x2<MODE == 0>(x, y, z, hi(sx), hi(sy), hi(sz), hi(nx), hi(ny), hi(nz), hi(cr),
+                                hi(ci), hi(dr), hi(di), hi(md), k2, kim2, thr2, CK, pa, pb, pi);
+      } else {
+        const float4 c = at(6, j), d = at(7, j);
+        pair_lap_x2<MODE == 0>(x, y, z, lo(sx), lo(sy), lo(sz), lo(nx), lo(ny), lo(nz), lo(c),
+                               lo(d), thr2, pa);
+        pair_lap_x2<MODE == 0>(x, y, z, hi(sx), hi(sy), hi(sz), hi(nx), hi(ny), hi(nz), hi(c),
+                               hi(d), thr2, pa);
+      }
+    }
+  }
+  outr = (pa.x - pb.x) + (pa.y - pb.y);
+  outi = pi.x + pi.y;
+}
+
+template <int KIND, bool CK, int MODE, int TILE>
+__device__ __forceinline__ void tile_eval(const TileSmem<KIND, double, TILE>& T, int j0, int j1,
+                                          double tx, double ty, double tz, double k, double kim,
+                                          double thr2, double& outr, double& outi,
+                                          const double2* tab) {
+  outr = outi = 0.0;
+#pragma unroll 4
+  for (int j = j0; j < j1; ++j) {
+    const double4 s = T.st[j];
+    if constexpr (MODE == 2)
+      pair_charge<KIND>(tx, ty, tz, T.g0[j], s, k, kim, CK, outr, outi, tab);
+    else if constexpr (KIND == 1)
+      pair_helm<MODE == 0>(tx, ty, tz, T.g0[j], T.g1[j], s, k, kim, thr2, CK, outr, outi, tab);
+    else
+      pair_lap<double, MODE == 0>(tx, ty, tz, T.g0[j], T.g1[j], make_double2(s.x, s.y), thr2, outr);
+  }
+}
+
+// Near lists of a leaf's targets (PROXYT = false) or proxy potentials of 128
+// of a node's proxies (PROXYT = true).  One barrier per tile: the tile is
+// double-buffered, and the next one's sources are already in registers.
+// FP32 is bound by the XU pipe (3 MUFU operations a pair; 68 % busy in the
+// leaves, 80 % in the proxies), FP64 by the FP64 pipe.  Far field of 146,016
+// Helmholtz nodes (320,312 sources): FP32 10.9 -> 9.6 ms, FP64 49.6 -> 42.3
+// (with pair.cuh's FP64 pair); 207,576 Laplace nodes: 6.9 -> 4.9 and 23.8 ->
+// 21.2.  Before, one source at a time in one buffer, the downward pass in
+// the same kernel, and a quarter to half of a leaf's warps idle.
 template <int KIND, typename R, bool CK, bool PROXYT>
-__global__ void __launch_bounds__(kEvThreads)
+__global__ void __launch_bounds__(kEvBlock<PROXYT>, (kEvMinBlocks<KIND, R, PROXYT>))
     tree_eval_kernel(TreeArgs ta, KParams kp, const R* __restrict__ str,
                      const R* __restrict__ qhat, R* __restrict__ phi,
                      double* __restrict__ partial, int nd) {
-  using R2 = typename Vec<R>::T2;
   using R4 = typename Vec<R>::T4;
   constexpr int SW = KIND == 1 ? 4 : 2;
   constexpr int C = KIND == 1 ? 2 : 1;
-  __shared__ R4 sg0[kEvTile];
-  __shared__ R2 sg1[kEvTile];
-  __shared__ R4 sst[kEvTile];
-  __shared__ R2 sphi[PROXYT ? 1 : tree::kMaxProxies];
-  __shared__ double2 stab[sizeof(R) == 8 && KIND == 1 ? kFarTrigN : 1];
+  constexpr int NT = kEvBlock<PROXYT>, TILE = NT, NW = NT / 32;
+  constexpr bool F32 = sizeof(R) == 4;
+  __shared__ __align__(16) TileSmem<KIND, R, TILE> tile[2];
+  __shared__ double2 stab[!F32 && KIND == 1 ? kFarTrigN : 1];
   const double2* tab = nullptr;
-  if constexpr (sizeof(R) == 8 && KIND == 1) {
-    fill_far_trig_table(stab);  // published by the first __syncthreads below
+  if constexpr (!F32 && KIND == 1) {
+    fill_far_trig_table(stab);
     tab = stab;
   }
   const int tid = threadIdx.x, m = blockIdx.y;
@@ -305,151 +507,201 @@ __global__ void __launch_bounds__(kEvThreads)
   const TNodeD tn = ta.tn[node];
   // FP32 shifts coordinates to the node centre; FP64 keeps them absolute so
   // that t - s of a close pair stays exact (as the direct far kernels do)
-  constexpr bool kShift = sizeof(R) == 4;
-  const double cx = kShift ? 0.5 * (tn.lo[0] + tn.hi[0]) : 0.0,
-               cy = kShift ? 0.5 * (tn.lo[1] + tn.hi[1]) : 0.0,
-               cz = kShift ? 0.5 * (tn.lo[2] + tn.hi[2]) : 0.0;
-  bool act, wact;  // this thread's / this warp's targets exist
+  const double cx = F32 ? 0.5 * (tn.lo[0] + tn.hi[0]) : 0.0,
+               cy = F32 ? 0.5 * (tn.lo[1] + tn.hi[1]) : 0.0,
+               cz = F32 ? 0.5 * (tn.lo[2] + tn.hi[2]) : 0.0;
+  // this thread's target and its part of every tile
+  const int nt = PROXYT ? min(NT, tn.np0 * tn.np1 * tn.np2 - int(k0)) : int(tn.e - tn.b);
+  const int tw = (nt + 31) / 32;            // warps of targets
+  const int parts = PROXYT ? 1 : NW / tw;   // parts of the tile
+  const int part = (tid >> 5) / tw;         // (parts or more: this warp only loads)
+  const int ti = tid - part * tw * 32;      // target of this thread
+  const bool act = ti < nt, work = part < parts;
   double x = cx, y = cy, z = cz;
-  if constexpr (PROXYT) {
-    const int64_t P = int64_t(tn.np0) * tn.np1 * tn.np2;
-    act = k0 + tid < P;
-    wact = k0 + (tid & ~31) < P;
-    if (act) {
-      const int64_t q = tn.tpoff + k0 + tid;
-      x = ta.tpx[q];
-      y = ta.tpy[q];
-      z = ta.tpz[q];
-    }
-  } else {
-    act = tn.b + tid < tn.e;
-    wact = tn.b + (tid & ~31) < tn.e;
-    if (act) {
-      const int64_t q = tn.b + tid;
-      x = ta.tx[q];
-      y = ta.ty[q];
-      z = ta.tz[q];
-    }
+  if (act) {
+    const int64_t q = PROXYT ? tn.tpoff + k0 + ti : tn.b + ti;
+    x = PROXYT ? ta.tpx[q] : ta.tx[q];
+    y = PROXYT ? ta.tpy[q] : ta.ty[q];
+    z = PROXYT ? ta.tpz[q] : ta.tz[q];
   }
   const R tx = R(x - cx), ty = R(y - cy), tz = R(z - cz);
   const R thr2 = R(kp.thresh * kp.thresh), k = R(kp.kr), kim = R(kp.ki);
   double accr = 0.0, acci = 0.0;
-  int n = node;
-  int64_t e0 = PROXYT ? tn.ce0 : tn.pe0, e1 = PROXYT ? tn.ce1 : tn.pe1;
-  const EntryD* ents = PROXYT ? ta.cent : ta.pent;
-  while (true) {
-    for (int64_t q = e0; q < e1; ++q) {
-      const EntryD en = ents[q];
-      for (int sb = en.b; sb < en.e; sb += kEvTile) {
-        const int ns = min(kEvTile, en.e - sb);
-        __syncthreads();
-        for (int qq = tid; qq < ns; qq += kEvThreads) {
-          const int s = sb + qq;
-          if (en.kind == 2) {
-            sg0[qq] = R4{R(ta.spx[s] - cx), R(ta.spy[s] - cy), R(ta.spz[s] - cz), R(0)};
-            const R* qp = qhat + (size_t(s) * nd + m) * C;
-            sst[qq] = R4{qp[0], C == 2 ? qp[C - 1] : R(0), R(0), R(0)};
-          } else {
-            sg0[qq] = R4{R(ta.sx[s] - cx), R(ta.sy[s] - cy), R(ta.sz[s] - cz), R(ta.snx[s])};
-            sg1[qq] = R2{R(ta.sny[s]), R(ta.snz[s])};
-            const R* sp = str + (size_t(s) * nd + m) * SW;
-            if constexpr (SW == 4)
-              sst[qq] = R4{sp[0], sp[1], sp[2], sp[3]};
-            else
-              sst[qq] = R4{sp[0], sp[1], R(0), R(0)};
-          }
-        }
-        __syncthreads();
-        R pr = R(0), pi = R(0);
-        if (!wact) {
-          // a warp without targets only helps load the tiles
-        } else if (en.kind == 2) {
-#pragma unroll 4
-          for (int j = 0; j < ns; ++j) pair_charge<KIND>(tx, ty, tz, sg0[j], sst[j], k, kim, CK, pr, pi, tab);
-        } else if (en.kind == 1) {
-#pragma unroll 4
-          for (int j = 0; j < ns; ++j) {
-            if constexpr (KIND == 1) {
-              pair_helm<false>(tx, ty, tz, sg0[j], sg1[j], sst[j], k, kim, thr2, CK, pr, pi, tab);
-            } else {
-              const R4 s = sst[j];
-              pair_lap<R, false>(tx, ty, tz, sg0[j], sg1[j], R2{s.x, s.y}, thr2, pr);
-            }
-          }
-        } else {
-#pragma unroll 4
-          for (int j = 0; j < ns; ++j) {
-            if constexpr (KIND == 1) {
-              pair_helm<true>(tx, ty, tz, sg0[j], sg1[j], sst[j], k, kim, thr2, CK, pr, pi, tab);
-            } else {
-              const R4 s = sst[j];
-              pair_lap<R, true>(tx, ty, tz, sg0[j], sg1[j], R2{s.x, s.y}, thr2, pr);
-            }
-          }
-        }
-        accr += double(pr);
-        acci += double(pi);
+  TileIter<PROXYT, TILE> it;
+  it.start(ta, node, tn);
+  RawSource<R> raw;
+  auto load = [&]() {
+    // past the entry's end: its last source without strength
+    const int s = min(it.sb + tid, it.en.e - 1);
+    const bool in = it.sb + tid < it.en.e;
+    if (it.en.kind == 2) {
+      raw.x = ta.spx[s], raw.y = ta.spy[s], raw.z = ta.spz[s];
+      raw.nx = raw.ny = raw.nz = 0.0;
+      const R* qp = qhat + (size_t(s) * nd + m) * C;
+      raw.s = in ? R4{qp[0], C == 2 ? qp[C - 1] : R(0), R(0), R(0)} : R4{R(0), R(0), R(0), R(0)};
+    } else {
+      raw.x = ta.sx[s], raw.y = ta.sy[s], raw.z = ta.sz[s];
+      raw.nx = ta.snx[s], raw.ny = ta.sny[s], raw.nz = ta.snz[s];
+      const R* sp = str + (size_t(s) * nd + m) * SW;
+      raw.s = R4{R(0), R(0), R(0), R(0)};
+      if (in) {
+        raw.s.x = sp[0], raw.s.y = sp[1];
+        if constexpr (SW == 4) raw.s.z = sp[2], raw.s.w = sp[3];
       }
     }
-    if (PROXYT) break;
-    n = ta.tn[n].parent;
-    if (n < 0) break;
-    e0 = ta.tn[n].pe0;
-    e1 = ta.tn[n].pe1;
-  }
-  if constexpr (!PROXYT) {
-    // downward pass: proxy potentials of the leaf's ancestors (and its own)
-    for (int a = node; a >= 0; a = ta.tn[a].parent) {
-      const TNodeD an = ta.tn[a];
-      if (an.tpoff < 0) continue;
-      const int P = an.np0 * an.np1 * an.np2;
-      __syncthreads();
-      for (int q = tid; q < P; q += kEvThreads) {
-        const R* pp = phi + (size_t(an.tpoff + q) * nd + m) * C;
-        sphi[q] = R2{pp[0], C == 2 ? pp[C - 1] : R(0)};
+  };
+  if (it.valid) load();
+  for (int b = 0; it.valid; b ^= 1) {
+    auto& T = tile[b];
+    if constexpr (F32) {
+      T.v[0][tid] = -R(raw.x - cx);
+      T.v[1][tid] = -R(raw.y - cy);
+      T.v[2][tid] = -R(raw.z - cz);
+      T.v[3][tid] = R(raw.nx);
+      T.v[4][tid] = R(raw.ny);
+      T.v[5][tid] = R(raw.nz);
+      T.v[6][tid] = raw.s.x;
+      T.v[7][tid] = raw.s.y;
+      if constexpr (SW == 4) {
+        T.v[8][tid] = raw.s.z;
+        T.v[9][tid] = raw.s.w;
       }
-      __syncthreads();
-      if (act) {
-        const double h0 = 0.5 * (an.hi[0] - an.lo[0]), h1 = 0.5 * (an.hi[1] - an.lo[1]),
-                     h2 = 0.5 * (an.hi[2] - an.lo[2]);
-        const R u0 = h0 > 0.0 ? R((x - 0.5 * (an.lo[0] + an.hi[0])) / h0) : R(0);
-        const R u1 = h1 > 0.0 ? R((y - 0.5 * (an.lo[1] + an.hi[1])) / h1) : R(0);
-        const R u2 = h2 > 0.0 ? R((z - 0.5 * (an.lo[2] + an.hi[2])) / h2) : R(0);
-        R Lx[kP], Ly[kP], Lz[kP];
-        lagrange(an.np0, u0, Lx);
-        lagrange(an.np1, u1, Ly);
-        lagrange(an.np2, u2, Lz);
-        R sr = R(0), si = R(0);
-        for (int i = 0; i < an.np0; ++i)
-          for (int j = 0; j < an.np1; ++j) {
-            const R w = Lx[i] * Ly[j];
-            const R2* ph = sphi + (i * an.np1 + j) * an.np2;
-            R tr = R(0), ti = R(0);
-#pragma unroll
-            for (int l = 0; l < kP; ++l)
-              if (l < an.np2) {
-                tr = fma(Lz[l], ph[l].x, tr);
-                ti = fma(Lz[l], ph[l].y, ti);
-              }
-            sr = fma(w, tr, sr);
-            si = fma(w, ti, si);
-          }
-        accr += double(sr);
-        acci += double(si);
-      }
+    } else {
+      T.g0[tid] = R4{raw.x, raw.y, raw.z, raw.nx};
+      T.g1[tid] = typename Vec<R>::T2{raw.ny, raw.nz};
+      T.st[tid] = raw.s;
+    }
+    const int kind = it.en.kind, ns = min(TILE, it.en.e - it.sb);
+    it.next();
+    if (it.valid) load();
+    __syncthreads();
+    if (work) {
+      // part p of the tile: a multiple of four sources
+      const int len = PROXYT ? TILE : ((ns + parts - 1) / parts + 3) & ~3;
+      const int j0 = part * len, j1 = min(j0 + len, F32 ? (ns + 3) & ~3 : ns);
+      R pr, pi;
+      auto go = [&](auto mode) {
+        constexpr int MODE = decltype(mode)::value;
+        if constexpr (F32)
+          tile_eval<KIND, CK, MODE, TILE>(T, j0, j1, tx, ty, tz, k, kim, thr2, pr, pi);
+        else
+          tile_eval<KIND, CK, MODE, TILE>(T, j0, j1, tx, ty, tz, k, kim, thr2, pr, pi, tab);
+      };
+      if (kind == 2)
+        go(std::integral_constant<int, 2>{});
+      else if (kind == 1)
+        go(std::integral_constant<int, 1>{});
+      else
+        go(std::integral_constant<int, 0>{});
+      accr += double(pr);
+      acci += double(pi);
     }
   }
-  if (!act) return;
   if constexpr (PROXYT) {
-    R* o = phi + (size_t(tn.tpoff + k0 + tid) * nd + m) * C;
+    if (!act) return;
+    R* o = phi + (size_t(tn.tpoff + k0 + ti) * nd + m) * C;
     o[0] = R(accr);
     if constexpr (C == 2) o[1] = R(acci);
   } else {
-    const int64_t it = ta.tperm[tn.b + tid];
-    double* o = partial + (size_t(it) * nd + m) * C;
-    o[0] = accr;
-    if constexpr (C == 2) o[1] = acci;
+    // the parts' sums, in order
+    if (parts > 1) {
+      double2* sred = reinterpret_cast<double2*>(tile);
+      static_assert(sizeof(tile) >= NT * sizeof(double2), "reduction buffer");
+      __syncthreads();
+      sred[tid] = make_double2(accr, acci);
+      __syncthreads();
+      for (int p = 1; p < parts; ++p)
+        if (part == 0) {
+          const double2 v = sred[tid + p * tw * 32];
+          accr += v.x;
+          acci += v.y;
+        }
+    }
+    if (!act || part != 0) return;
+    const int64_t o = (size_t(ta.tperm[tn.b + ti]) * nd + m) * C;
+    partial[o] = accr;
+    if constexpr (C == 2) partial[o + 1] = acci;
   }
+}
+
+// Downward pass: the proxy potentials of a leaf and its ancestors
+// interpolated to its targets, added to the near lists' sums.  LZ: compiled
+// bound of the grid's points along the third side.
+template <typename R, int LZ>
+__device__ __forceinline__ void down_node(const R* Lx, const R* Ly, const R* Lz, int np0, int np1,
+                                          int np2, const typename Vec<R>::T2* ph, R& outr,
+                                          R& outi) {
+  R sr = R(0), si = R(0);
+#pragma unroll
+  for (int i = 0; i < kP; ++i) {
+    if (i >= np0) break;
+#pragma unroll
+    for (int j = 0; j < kP; ++j) {
+      if (j >= np1) break;
+      const R w = Lx[i] * Ly[j];
+      R tr = R(0), ti = R(0);
+#pragma unroll
+      for (int l = 0; l < LZ; ++l)
+        if (l < np2) {
+          tr = fma(Lz[l], ph[l].x, tr);
+          ti = fma(Lz[l], ph[l].y, ti);
+        }
+      sr = fma(w, tr, sr);
+      si = fma(w, ti, si);
+      ph += np2;
+    }
+  }
+  outr = sr;
+  outi = si;
+}
+
+template <typename R, int C>
+__global__ void __launch_bounds__(kEvThreads)
+    tree_down_kernel(TreeArgs ta, const R* __restrict__ phi, double* __restrict__ partial, int nd) {
+  using R2 = typename Vec<R>::T2;
+  __shared__ R2 sphi[tree::kMaxProxies];
+  const int tid = threadIdx.x, m = blockIdx.y;
+  const int node = ta.leaves[blockIdx.x];
+  const int64_t b = ta.tn[node].b;
+  const bool act = b + tid < ta.tn[node].e;
+  double x = 0.0, y = 0.0, z = 0.0, accr = 0.0, acci = 0.0;
+  if (act) x = ta.tx[b + tid], y = ta.ty[b + tid], z = ta.tz[b + tid];
+  bool any = false;
+  for (int a = node; a >= 0; a = ta.tn[a].parent) {
+    const TNodeD an = ta.tn[a];
+    if (an.tpoff < 0) continue;
+    any = true;
+    const int P = an.np0 * an.np1 * an.np2;
+    __syncthreads();
+    for (int q = tid; q < P; q += kEvThreads) {
+      const R* pp = phi + (size_t(an.tpoff + q) * nd + m) * C;
+      sphi[q] = R2{pp[0], C == 2 ? pp[C - 1] : R(0)};
+    }
+    __syncthreads();
+    if (!act) continue;
+    const double h0 = 0.5 * (an.hi[0] - an.lo[0]), h1 = 0.5 * (an.hi[1] - an.lo[1]),
+                 h2 = 0.5 * (an.hi[2] - an.lo[2]);
+    const R u0 = h0 > 0.0 ? R((x - 0.5 * (an.lo[0] + an.hi[0])) / h0) : R(0);
+    const R u1 = h1 > 0.0 ? R((y - 0.5 * (an.lo[1] + an.hi[1])) / h1) : R(0);
+    const R u2 = h2 > 0.0 ? R((z - 0.5 * (an.lo[2] + an.hi[2])) / h2) : R(0);
+    R Lx[kP], Ly[kP], Lz[kP];
+    lagrange(an.np0, u0, Lx);
+    lagrange(an.np1, u1, Ly);
+    lagrange(an.np2, u2, Lz);
+    R sr, si;
+    if (an.np2 <= 4)
+      down_node<R, 4>(Lx, Ly, Lz, an.np0, an.np1, an.np2, sphi, sr, si);
+    else if (an.np2 <= 8)
+      down_node<R, 8>(Lx, Ly, Lz, an.np0, an.np1, an.np2, sphi, sr, si);
+    else
+      down_node<R, kP>(Lx, Ly, Lz, an.np0, an.np1, an.np2, sphi, sr, si);
+    accr += double(sr);
+    acci += double(si);
+  }
+  if (!act || !any) return;
+  const size_t o = (size_t(ta.tperm[b + tid]) * nd + m) * C;
+  partial[o] += accr;
+  if constexpr (C == 2) partial[o + 1] += acci;
 }
 
 // Several densities per block (MD of them, densities m0 .. m0 + MD - 1 on
@@ -474,17 +726,19 @@ __global__ void __launch_bounds__(kEvThreads)
   __shared__ R4 sg0[kMdTile];
   __shared__ R2 sg1[kMdTile];
   __shared__ R4 sab[kMdTile];  // (a_s, b_s) of particle sources
-  // the densities (or proxy charges) of the list phase and the proxy
-  // potentials of the downward phase share one buffer
+  // the list phase's densities (or proxy charges) and sine/cosine table
+  // share one buffer with the downward phase's proxy potentials
+  constexpr bool kTab = sizeof(R) == 8 && KIND == 1;
   constexpr size_t kSstBytes = sizeof(R) * kMdTile * MD * C;
+  constexpr size_t kListBytes = kSstBytes + (kTab ? sizeof(double2) * kFarTrigN : 0);
   constexpr size_t kPhiBytes = PROXYT ? 0 : sizeof(R2) * tree::kMaxProxies;
-  __shared__ __align__(16) unsigned char sbuf[kSstBytes > kPhiBytes ? kSstBytes : kPhiBytes];
+  __shared__ __align__(16) unsigned char sbuf[kListBytes > kPhiBytes ? kListBytes : kPhiBytes];
   R(*sst)[MD][C] = reinterpret_cast<R(*)[MD][C]>(sbuf);
   R2* sphi = reinterpret_cast<R2*>(sbuf);
-  __shared__ double2 stab[sizeof(R) == 8 && KIND == 1 ? kFarTrigN : 1];
   const double2* tab = nullptr;
-  if constexpr (sizeof(R) == 8 && KIND == 1) {
-    fill_far_trig_table(stab);  // published by the first __syncthreads below
+  if constexpr (kTab) {
+    double2* stab = reinterpret_cast<double2*>(sbuf + kSstBytes);
+    fill_far_trig_table(stab);
     tab = stab;
   }
   const int tid = threadIdx.x;
@@ -752,13 +1006,17 @@ cudaError_t run_t(const TreeArgs& ta, const KParams& kp, int nup, const UpItemD*
   } else {
     if (npitems > 0) {
       tree_eval_kernel<KIND, R, CK, true>
-          <<<dim3(unsigned(npitems), 1u), kEvThreads, 0, st>>>(ta, kp, str, qhat, phi, partial, nd);
+          <<<dim3(unsigned(npitems), 1u), kEvBlock<true>, 0, st>>>(ta, kp, str, qhat, phi, partial, nd);
       ++launches;
     }
     if (nleaf > 0) {
       tree_eval_kernel<KIND, R, CK, false>
-          <<<dim3(unsigned(nleaf), 1u), kEvThreads, 0, st>>>(ta, kp, str, qhat, phi, partial, nd);
+          <<<dim3(unsigned(nleaf), 1u), kEvBlock<false>, 0, st>>>(ta, kp, str, qhat, phi, partial, nd);
       ++launches;
+      if (npitems > 0) {
+        tree_down_kernel<R, C><<<dim3(unsigned(nleaf), 1u), kEvThreads, 0, st>>>(ta, phi, partial, nd);
+        ++launches;
+      }
     }
   }
   note_launches(launches);

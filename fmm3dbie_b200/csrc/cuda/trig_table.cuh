@@ -43,36 +43,79 @@ __device__ __forceinline__ void sincos_tab(double x, const double2* tab, double&
 
 // The far-field variant of the same method, for the direct and hierarchical
 // far-field kernels, whose phases stay below 100 and whose products only need
-// ~1e-14: the same 256-entry table and series, with j found by the
-// round-to-integer of adding 1.5 * 2^52 (no conversion instructions) and the
-// reduction x - j (2 pi / N) in one fused multiply-add with 2 pi / N rounded
-// to FP64: its error, j times the rounding of the step (at most 1.7e-18), is
-// below 1e-14 for x < 100.
-constexpr int kFarTrigN = kTrigN;
-constexpr double kRoundMagic = 6755399441055744.0;  // 1.5 * 2^52
+// ~1e-14.  The FP64 pipe bounds those kernels, so the phase goes straight to
+// table steps and the table is fine enough for short series:
+//   u = k r N / (2 pi) = j + f, |f| <= 1/2, j by the round-to-integer of adding
+//   1.5 * 2^52 (no conversion instructions), f = u - j in one fused
+//   multiply-add (its error is the rounding of k N / (2 pi): 1.1e-16 of the
+//   phase);
+//   sin(2 pi f / N) to f^3, with the f^5 term economised on |f| <= 1/2
+//   (Lanczos: x^5 ~ 5/4 h^2 x^3 - 5/16 h^4 x on |x| <= h, error h^5 / 16), which
+//   leaves h^5 / 1920 = 1.4e-16 for h = pi / 1024; cos to f^4 (next term
+//   1.2e-18).
+// 12 FP64 operations; 256 entries with the series to rho^5 and rho^6 and a
+// separate phase k r took 15.
+constexpr int kFarTrigN = 1024;
+constexpr double kFarTrigInvStep = 162.97466172610083;  // 1024 / (2 pi)
+constexpr double kRoundMagic = 6755399441055744.0;      // 1.5 * 2^52
+constexpr double kFarTrigStep = 0.006135923151542565;   // 2 pi / 1024
+constexpr double kFarTrigH = 0.5 * kFarTrigStep;
+constexpr double kFarS1 =
+    kFarTrigStep * (1.0 - 5.0 / 16.0 / 120.0 * kFarTrigH * kFarTrigH * kFarTrigH * kFarTrigH);
+constexpr double kFarS3 = kFarTrigStep * kFarTrigStep * kFarTrigStep *
+                          (-1.0 / 6.0 + 5.0 / 4.0 / 120.0 * kFarTrigH * kFarTrigH);
+constexpr double kFarC2 = -0.5 * kFarTrigStep * kFarTrigStep;
+constexpr double kFarC4 = kFarTrigStep * kFarTrigStep * kFarTrigStep * kFarTrigStep / 24.0;
 
-__device__ __forceinline__ void fill_far_trig_table(double2* tab) { fill_trig_table(tab); }
+// Fills tab[q] = (cos, sin)(2 pi q / N): the first octant by sincos (one
+// value a thread for 128 threads), the others by symmetry.  Ends with a
+// barrier.
+__device__ __forceinline__ void fill_far_trig_table(double2* tab) {
+  constexpr int E = kFarTrigN / 8;
+  for (int q = threadIdx.x; q <= E; q += blockDim.x) {
+    double s, c;
+    sincospi(double(q) / (kFarTrigN / 2), &s, &c);
+    tab[q] = make_double2(c, s);
+  }
+  __syncthreads();
+  for (int q = E + 1 + threadIdx.x; q < kFarTrigN; q += blockDim.x) {
+    const int o = q / E, r = q % E;
+    const double2 t = tab[o & 1 ? E - r : r];  // entries 0 .. E only
+    const double c = o & 1 ? t.y : t.x, s = o & 1 ? t.x : t.y;  // within the quadrant
+    const int quad = o >> 1;
+    tab[q] = quad == 0   ? make_double2(c, s)
+             : quad == 1 ? make_double2(-s, c)
+             : quad == 2 ? make_double2(-c, -s)
+                         : make_double2(s, -c);
+  }
+  __syncthreads();
+}
 
-__device__ __forceinline__ void sincos_far(double x, const double2* tab, double& s, double& c) {
-  const double u = fma(x, kTrigInvStep, kRoundMagic);  // 1.5 2^52 + rint(x / step)
+// sin and cos of k r, kstep = k N / (2 pi).
+__device__ __forceinline__ void sincos_far(double r, double kstep, const double2* tab, double& s,
+                                           double& c) {
+  const double u = fma(r, kstep, kRoundMagic);
   const int j = __double2loint(u) & (kFarTrigN - 1);
-  const double jd = u - kRoundMagic;
-  const double rho = fma(-jd, kTrigStep, x);
-  const double r2 = rho * rho;
-  const double sp = fma(rho * r2, fma(r2, 1.0 / 120.0, -1.0 / 6.0), rho);
-  const double cp = fma(r2, fma(r2, fma(r2, -1.0 / 720.0, 1.0 / 24.0), -0.5), 1.0);
+  const double f = fma(r, kstep, kRoundMagic - u);
+  const double f2 = f * f;
+  const double sp = f * fma(f2, kFarS3, kFarS1);
+  const double cp = fma(f2, fma(f2, kFarC4, kFarC2), 1.0);
   const double2 t = tab[j];
   s = fma(t.y, cp, t.x * sp);
   c = fma(t.x, cp, -(t.y * sp));
 }
 
-// 1/sqrt(a) in FP64 for a > 0 in the FP32 normal range: the FP32 hardware
-// approximation y0 (relative error e0 ~ 2^-22) refined by one third-order
-// step of the binomial series of (1 - e)^(-1/2), e = 1 - a y0^2:
+// 1/sqrt(a) in FP64 for normal a > 0: the hardware's FP64 approximation y0
+// (rsqrt.approx.ftz.f64, relative error e0 / 2 with e0 = 1 - a y0^2 about
+// 2^-20) refined by one third-order step of the binomial series of
+// (1 - e)^(-1/2):
 //   y = y0 (1 + e/2 + 3 e^2 / 8),
-// whose truncation error 5 e^3 / 16 ~ 1e-20 is below the FP64 rounding.
+// whose truncation error 5 e^3 / 16 is below the FP64 rounding.  Starting
+// from the FP32 approximation took two conversions more, on the pipe that
+// the approximation itself uses.
 __device__ __forceinline__ double rsqrt_far(double a) {
-  const double y0 = double(rsqrtf(float(a)));
+  double y0;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(a));
   const double e = fma(-(a * y0), y0, 1.0);
   return fma(y0 * e, fma(e, 0.375, 0.5), y0);
 }
