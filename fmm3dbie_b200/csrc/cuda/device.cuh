@@ -176,6 +176,7 @@ struct Segs {
   const int64_t* chunk_hi = nullptr;    // device, nchunk: one past its last node
   const int32_t* seg_chunk0 = nullptr;  // device, nseg+1: first chunk of each segment
   const int32_t* node_seg = nullptr;    // device, npts: segment of each node (null if nseg == 1)
+  int* ticket = nullptr;                // device: counter of finished blocks, 0 between launches
 };
 // out[2*(k*nsys + sys)] + i out[2*(k*nsys + sys)+1] = sum over sys's nodes of
 // wts * conj(V_k) w, for k < m, V_k = V + k*ldv; partial needs
@@ -183,9 +184,6 @@ struct Segs {
 cudaError_t launch_mdot(const double* V, int64_t ldv, int m, const double* w, const double* wts,
                         int nd, int cplx, const Segs& sg, double* partial, double* out,
                         cudaStream_t st);
-// w[e] -= sum_k h[k, sys(e)] V_k[e]   (h complex on device, layout as out)
-cudaError_t launch_maxpy(const double* V, int64_t ldv, int m, const double* h, double* w,
-                         int64_t n, int nd, int cplx, const Segs& sg, cudaStream_t st);
 // y[e] = s[sys(e)] x[e], s complex on device (y may alias x)
 cudaError_t launch_dscale(const double* x, double* y, const double* s, int64_t n, int nd,
                           int cplx, const Segs& sg, cudaStream_t st);
@@ -195,17 +193,34 @@ cudaError_t launch_axpby(const double* x, double* y, double ar, double ai, doubl
 // y[e] = a[sys(e)] x[e] + b y[e], a complex per system on device
 cudaError_t launch_axpbys(const double* x, double* y, const double* a, double br, double bi,
                           int64_t n, int nd, int cplx, const Segs& sg, cudaStream_t st);
-// GMRES least squares on the device, FP64, one thread per system: the
-// Givens step of iteration it (Hessenberg column from the two Gram-Schmidt
-// passes h1, h2 and the new vector's squared norm nrm, rotations, residual
-// estimate, stopping test, scale = 1/||w|| for the systems that go on), and
-// the back-substitution into the combination coefficients.  H (M+1) x M per
-// system, column-major; cs, sn M, sv M+1 per system; all complex (re, im).
-cudaError_t launch_gmres_givens(int it, int M, int nsys, const double* h1, const double* h2,
-                                const double* nrm, const double* zid, double* H, double* cs,
-                                double* sn, double* sv, const double* bnorm, const double* eps,
-                                int64_t* done, int* brk, double* errs, double* scale,
-                                cudaStream_t st);
+// GMRES least squares on the device, FP64: the Givens step of iteration it
+// (Hessenberg column from the two Gram-Schmidt passes h1, h2 and the new
+// vector's squared norm nrm, rotations, residual estimate, stopping test,
+// scale = 1/||w|| for the systems that go on), and the back-substitution into
+// the combination coefficients.  H (M+1) x M per system, column-major; cs,
+// sn M, sv M+1 per system; all complex (re, im).
+struct GivensArgs {
+  int it = 0, M = 0, nsys = 0;
+  const double *h1 = nullptr, *h2 = nullptr, *nrm = nullptr, *zid = nullptr;
+  double *H = nullptr, *cs = nullptr, *sn = nullptr, *sv = nullptr;
+  const double *bnorm = nullptr, *eps = nullptr;
+  int64_t* done = nullptr;
+  int* brk = nullptr;
+  double *errs = nullptr, *scale = nullptr;
+};
+// One pass of the orthogonalisation: w -= sum_k hsub[k] Vsub_k for k < msub
+// (if hsub), then out = the inner products of launch_mdot with the m vectors
+// V_k of the new w (V may be w), then the Givens step gv (if given; gv->nrm is
+// out).
+cudaError_t launch_orth(const double* V, int64_t ldv, int m, double* w, const double* wts, int nd,
+                        int cplx, const Segs& sg, double* partial, double* out,
+                        const double* hsub, int msub, const double* Vsub, const GivensArgs* gv,
+                        cudaStream_t st);
+// State at the start of a solve from the squared norms of the residual and
+// (with an initial guess) of the right-hand side.
+cudaError_t launch_gmres_init(int M, int nsys, const double* nrm, const double* nrmb,
+                              double* scale, double* sv, double* bnorm, int64_t* done, int* brk,
+                              cudaStream_t st);
 cudaError_t launch_gmres_backsolve(int M, int nsys, int mused, const double* H, const double* sv,
                                    const int64_t* done, double* coef, cudaStream_t st);
 // Krylov-basis coefficients (mcols per system) of each system's GMRES

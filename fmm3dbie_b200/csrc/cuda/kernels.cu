@@ -1298,17 +1298,177 @@ __device__ __forceinline__ int sys_of(const Segs& sg, int64_t e, int nd) {
   return seg * nd + int(e - pt * nd);
 }
 
-// partial[((k*nd + d)*nchunk + c)] = sum over chunk c of wts * conj(V_k) w
-template <int CPLX>
-__global__ void mdot_partial_kernel(const double* __restrict__ V, int64_t ldv, int m,
-                                    const double* __restrict__ w, const double* __restrict__ wts,
-                                    int nd, Segs sg, double* __restrict__ partial) {
+// Complex values as (re, im) pairs.
+struct Z {
+  double r, i;
+};
+__device__ __forceinline__ Z zmul(Z a, Z b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
+__device__ __forceinline__ Z zadd(Z a, Z b) { return {a.r + b.r, a.i + b.i}; }
+__device__ __forceinline__ Z zconj(Z a) { return {a.r, -a.i}; }
+__device__ __forceinline__ Z zdiv(Z a, Z b) {
+  const double d = b.r * b.r + b.i * b.i;
+  return {(a.r * b.r + a.i * b.i) / d, (a.i * b.r - a.r * b.i) / d};
+}
+__device__ __forceinline__ Z zld(const double* p) { return {p[0], p[1]}; }
+__device__ __forceinline__ void zst(double* p, Z v) {
+  p[0] = v.r;
+  p[1] = v.i;
+}
+__device__ __forceinline__ Z zshfl(Z v, int lane) {
+  return {__shfl_sync(0xffffffffu, v.r, lane), __shfl_sync(0xffffffffu, v.i, lane)};
+}
+
+// Iteration it of system q, by one warp: the new Hessenberg column
+// H(0..it, it) = h1 + h2 (the two Gram-Schmidt passes) with zid on the
+// diagonal, the previous Givens rotations applied, the new rotation
+// (zrotmat_gmres, rotmat_gmres.f:60-100) against the norm of the new
+// vector, the rotated residual vector s, the residual estimate
+// |s(it+1)| / ||rhs||, and the stopping test; scale = 1/||w|| for the
+// systems that go on (0 for the others).  done[q]: 0 active, > 0 iterations
+// taken, < 0 zero right-hand side; brk[q] = 1 on a NaN (breakdown).
+// The lanes load 32 rotations and column entries at a time and the chain
+// runs through shuffles: with one thread a system every step waited for its
+// own stores and loads (7-12 us an iteration, now 2-3).
+__device__ __forceinline__ void givens_step(const GivensArgs& g, int q, int lane) {
+  const int it = g.it, M = g.M, nsys = g.nsys;
+  if (lane == 0) {
+    g.scale[2 * q] = 0.0;
+    g.scale[2 * q + 1] = 0.0;
+  }
+  if (g.done[q] != 0) return;
+  double* Hq = g.H + 2 * (size_t(q) * M + it) * (M + 1);  // column it of system q
+  double* cq = g.cs + 2 * size_t(q) * M;
+  double* sq = g.sn + 2 * size_t(q) * M;
+  double* vq = g.sv + 2 * size_t(q) * (M + 1);
+  auto column = [&](int k) {
+    const size_t o = 2 * (size_t(k) * nsys + q);
+    Z h = zadd(zld(g.h1 + o), zld(g.h2 + o));
+    if (k == it) h = zadd(h, zld(g.zid + 2 * q));
+    return h;
+  };
+  Z a = column(0);  // entry k as the rotations before k left it
+  for (int base = 0; base < it; base += 32) {
+    const int k = base + lane;
+    Z c{0, 0}, s{0, 0}, h{0, 0}, mine{0, 0};
+    if (k < it) {
+      c = zld(cq + 2 * k);
+      s = zld(sq + 2 * k);
+      h = column(k + 1);
+    }
+    const int n = min(32, it - base);
+    for (int j = 0; j < n; ++j) {
+      const Z cj = zshfl(c, j), sj = zshfl(s, j), b = zshfl(h, j);
+      const Z out = zadd(zmul(cj, a), zmul(zconj(sj), b));
+      const Z ms = {-sj.r, -sj.i};
+      a = zadd(zmul(ms, a), zmul(cj, b));
+      if (lane == j) mine = out;
+    }
+    if (k < it) zst(Hq + 2 * k, mine);
+  }
+  if (lane != 0) return;
+  const double wnrm = sqrt(fmax(g.nrm[2 * q], 0.0));
+  Z c, s;
+  if (a.r == 0.0 && a.i == 0.0) {
+    c = {0.0, 0.0};
+    s = {1.0, 0.0};
+  } else {
+    const Z t = zdiv(Z{wnrm, 0.0}, a);
+    const double cr = 1.0 / sqrt(1.0 + t.r * t.r + t.i * t.i);
+    c = {cr, 0.0};
+    s = {t.r * cr, t.i * cr};
+  }
+  zst(cq + 2 * it, c);
+  zst(sq + 2 * it, s);
+  zst(Hq + 2 * it, zadd(zmul(c, a), zmul(zconj(s), Z{wnrm, 0.0})));
+  const Z v = zld(vq + 2 * it);
+  const Z vn = {-(s.r * v.r - s.i * v.i), -(s.r * v.i + s.i * v.r)};
+  zst(vq + 2 * (it + 1), vn);
+  zst(vq + 2 * it, zmul(c, v));
+  const double err = g.bnorm[q] > 0.0 ? sqrt(vn.r * vn.r + vn.i * vn.i) / g.bnorm[q] : 0.0;
+  g.errs[size_t(q) * (M + 1) + it] = err;
+  if (!(err == err) || !(wnrm == wnrm)) {
+    g.brk[q] = 1;
+    g.done[q] = it + 1;
+    return;
+  }
+  // the new Krylov vector is normalised also when the system stops here: it
+  // is the last vector of the basis that carries the residual vector
+  if (wnrm > 0.0) g.scale[2 * q] = 1.0 / wnrm;
+  if (err <= g.eps[q] || it == M - 1 || wnrm == 0.0) g.done[q] = it + 1;
+}
+
+__global__ void gmres_givens_kernel(GivensArgs g) {
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q < g.nsys) givens_step(g, q, threadIdx.x & 31);
+}
+
+// out[2 b] = sum over the segment's chunks of the partials of b = (k, sys),
+// by one warp.
+__device__ __forceinline__ void reduce_dot(const double* partial, int nd, const Segs& sg, int b,
+                                           double* out, int lane) {
+  const int nsys = sg.nseg * nd;
+  const int k = b / nsys, sys = b - k * nsys;
+  const int seg = sys / nd, d = sys - seg * nd;
+  const size_t base = (size_t(k) * nd + d) * sg.nchunk;
+  double sr = 0, si = 0;
+  for (int c = sg.seg_chunk0[seg] + lane; c < sg.seg_chunk0[seg + 1]; c += 32) {
+    const double2 v = __ldcg(reinterpret_cast<const double2*>(partial) + base + c);
+    sr += v.x;
+    si += v.y;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    sr += __shfl_xor_sync(0xffffffffu, sr, off);
+    si += __shfl_xor_sync(0xffffffffu, si, off);
+  }
+  if (lane == 0) {
+    out[2 * b] = sr;
+    out[2 * b + 1] = si;
+  }
+}
+
+// One pass of the orthogonalisation over a chunk of nodes: w -= sum_k
+// hsub[k] V_k (if hsub), then the chunk's part of conj(V_k) w for the m
+// vectors V_k (V may be w).  FUSED: the last block to finish sums the chunks
+// and, with gv.nsys > 0, takes the Givens step, so that a Gram-Schmidt pass
+// is one launch instead of three.  (partial[((k*nd + d)*nchunk + c)] = the
+// sum over chunk c.)
+template <int CPLX, bool FUSED>
+__global__ void orth_kernel(const double* V, int64_t ldv, int m, double* w,
+                            const double* __restrict__ wts, int nd, Segs sg, double* partial,
+                            double* out, const double* __restrict__ hsub, int msub,
+                            const double* __restrict__ Vsub, GivensArgs gv) {
   __shared__ double2 red[256];
+  __shared__ int s_last;
   const int tid = threadIdx.x;
   const int rows = blockDim.x / nd;  // blockDim.x is a multiple of nd
   const int dd = tid % nd, r = tid / nd;
   const int c = blockIdx.x;
   const int64_t lo = sg.chunk_lo[c], hi = sg.chunk_hi[c];
+  if (hsub) {
+    const int nsys = sg.nseg * nd;
+    for (int64_t e = lo * nd + tid; e < hi * nd; e += blockDim.x) {
+      const int sy = sys_of(sg, e, nd);
+      if (CPLX) {
+        double2 x = reinterpret_cast<const double2*>(w)[e];
+#pragma unroll 4
+        for (int k = 0; k < msub; ++k) {
+          const double2 h = reinterpret_cast<const double2*>(hsub)[size_t(k) * nsys + sy];
+          const double2 v = reinterpret_cast<const double2*>(Vsub + size_t(k) * ldv)[e];
+          x.x -= h.x * v.x - h.y * v.y;
+          x.y -= h.x * v.y + h.y * v.x;
+        }
+        reinterpret_cast<double2*>(w)[e] = x;
+      } else {
+        double x = w[e];
+#pragma unroll 4
+        for (int k = 0; k < msub; ++k)
+          x -= hsub[2 * (size_t(k) * nsys + sy)] * Vsub[size_t(k) * ldv + e];
+        w[e] = x;
+      }
+    }
+    __syncthreads();
+  }
   if (32 % nd == 0) {
     // nd divides the warp: each warp takes whole vectors k = warp, warp + nw,
     // ... over the chunk (lane = row (lane / nd), density lane % nd), sums
@@ -1319,6 +1479,7 @@ __global__ void mdot_partial_kernel(const double* __restrict__ V, int64_t ldv, i
     for (int k = warp; k < m; k += nw) {
       const double* v = V + size_t(k) * ldv;
       double sr = 0, si = 0;
+#pragma unroll 2
       for (int64_t pt = lo + lr; pt < hi; pt += wr) {
         const int64_t e = pt * nd + ld;
         const double wt = wts[pt];
@@ -1340,23 +1501,21 @@ __global__ void mdot_partial_kernel(const double* __restrict__ V, int64_t ldv, i
         partial[2 * o + 1] = si;
       }
     }
-    return;
-  }
-  for (int k = 0; k < m; ++k) {
-    const double* v = V + size_t(k) * ldv;
-    double sr = 0, si = 0;
-    for (int64_t pt = lo + r; pt < hi; pt += rows) {
-      const int64_t e = pt * nd + dd;
-      const double wt = wts[pt];
-      if (CPLX) {
-        const double vr = v[2 * e], vi = v[2 * e + 1], xr = w[2 * e], xi = w[2 * e + 1];
-        sr += wt * (vr * xr + vi * xi);
-        si += wt * (vr * xi - vi * xr);
-      } else {
-        sr += wt * v[e] * w[e];
+  } else {
+    for (int k = 0; k < m; ++k) {
+      const double* v = V + size_t(k) * ldv;
+      double sr = 0, si = 0;
+      for (int64_t pt = lo + r; pt < hi; pt += rows) {
+        const int64_t e = pt * nd + dd;
+        const double wt = wts[pt];
+        if (CPLX) {
+          const double vr = v[2 * e], vi = v[2 * e + 1], xr = w[2 * e], xi = w[2 * e + 1];
+          sr += wt * (vr * xr + vi * xi);
+          si += wt * (vr * xi - vi * xr);
+        } else {
+          sr += wt * v[e] * w[e];
+        }
       }
-    }
-    {
       red[tid] = make_double2(sr, si);
       __syncthreads();
       if (tid < nd) {
@@ -1370,6 +1529,24 @@ __global__ void mdot_partial_kernel(const double* __restrict__ V, int64_t ldv, i
         partial[2 * o + 1] = ai;
       }
       __syncthreads();
+    }
+  }
+  if constexpr (FUSED) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(sg.ticket, 1) == int(gridDim.x) - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (tid == 0) *sg.ticket = 0;  // for the next launch
+    const int warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    if (warp < nw) {  // whole warps only
+      for (int b = warp; b < m * sg.nseg * nd; b += nw) reduce_dot(partial, nd, sg, b, out, lane);
+    }
+    if (gv.nsys > 0) {
+      __syncthreads();
+      if (warp < nw)
+        for (int q = warp; q < gv.nsys; q += nw) givens_step(gv, q, lane);
     }
   }
 }
@@ -1411,33 +1588,6 @@ __global__ void mdot_final_kernel(const double* __restrict__ partial, int nd, Se
     if (lane == 0) {
       out[2 * b] = sr;
       out[2 * b + 1] = si;
-    }
-  }
-}
-
-// w[e] -= sum_k h[k, sys(e)] V_k[e]
-template <int CPLX>
-__global__ void maxpy_kernel(const double* __restrict__ V, int64_t ldv, int m,
-                             const double* __restrict__ h, double* __restrict__ w, int64_t n,
-                             int nd, Segs sg) {
-  const int nsys = sg.nseg * nd;
-  for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
-       e += int64_t(gridDim.x) * blockDim.x) {
-    const int sy = sys_of(sg, e, nd);
-    if (CPLX) {
-      double xr = w[2 * e], xi = w[2 * e + 1];
-      for (int k = 0; k < m; ++k) {
-        const double hr = h[2 * (k * nsys + sy)], hi = h[2 * (k * nsys + sy) + 1];
-        const double vr = V[size_t(k) * ldv + 2 * e], vi = V[size_t(k) * ldv + 2 * e + 1];
-        xr -= hr * vr - hi * vi;
-        xi -= hr * vi + hi * vr;
-      }
-      w[2 * e] = xr;
-      w[2 * e + 1] = xi;
-    } else {
-      double x = w[e];
-      for (int k = 0; k < m; ++k) x -= h[2 * (k * nsys + sy)] * V[size_t(k) * ldv + e];
-      w[e] = x;
     }
   }
 }
@@ -2230,30 +2380,52 @@ cudaError_t launch_reduce_partials(int kind, const double* partial, int nchunks,
   return cudaGetLastError();
 }
 
-cudaError_t launch_mdot(const double* V, int64_t ldv, int m, const double* w, const double* wts,
-                        int nd, int cplx, const Segs& sg, double* partial, double* out,
+// Chunk sums times outputs that the last block of orth_kernel takes itself
+// (16 bytes each, read by one SM: 128 KB, about 2 us, the price of the
+// launch it saves); larger reductions go to mdot_final_kernel.
+constexpr int64_t kFusedReduce = 8192;
+
+cudaError_t launch_orth(const double* V, int64_t ldv, int m, double* w, const double* wts, int nd,
+                        int cplx, const Segs& sg, double* partial, double* out,
+                        const double* hsub, int msub, const double* Vsub, const GivensArgs* gv,
                         cudaStream_t st) {
   if (m <= 0) return cudaSuccess;
   if (nd < 1 || nd > 256) return cudaErrorInvalidValue;
   const int threads = (256 / nd) * nd;
+  // the fused tail works in whole warps
+  const bool fused = int64_t(m) * nd * sg.nchunk <= kFusedReduce && sg.ticket && threads >= 32;
+  GivensArgs none;
+  const GivensArgs& g = gv && fused ? *gv : none;
+  auto go = [&](auto kern) {
+    kern<<<sg.nchunk, threads, 0, st>>>(V, ldv, m, w, wts, nd, sg, partial, out, hsub, msub, Vsub,
+                                        g);
+  };
+  if (fused) {
+    if (cplx)
+      go(orth_kernel<1, true>);
+    else
+      go(orth_kernel<0, true>);
+    count();
+    return cudaGetLastError();
+  }
   if (cplx)
-    mdot_partial_kernel<1><<<sg.nchunk, threads, 0, st>>>(V, ldv, m, w, wts, nd, sg, partial);
+    go(orth_kernel<1, false>);
   else
-    mdot_partial_kernel<0><<<sg.nchunk, threads, 0, st>>>(V, ldv, m, w, wts, nd, sg, partial);
+    go(orth_kernel<0, false>);
   mdot_final_kernel<<<m * sg.nseg * nd, 256, 0, st>>>(partial, nd, sg, out);
   count(2);
+  if (gv) {
+    gmres_givens_kernel<<<(gv->nsys + 3) / 4, 128, 0, st>>>(*gv);
+    count();
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_maxpy(const double* V, int64_t ldv, int m, const double* h, double* w,
-                         int64_t n, int nd, int cplx, const Segs& sg, cudaStream_t st) {
-  if (m <= 0) return cudaSuccess;
-  if (cplx)
-    maxpy_kernel<1><<<grid_for(n, 256), 256, 0, st>>>(V, ldv, m, h, w, n, nd, sg);
-  else
-    maxpy_kernel<0><<<grid_for(n, 256), 256, 0, st>>>(V, ldv, m, h, w, n, nd, sg);
-  count();
-  return cudaGetLastError();
+cudaError_t launch_mdot(const double* V, int64_t ldv, int m, const double* w, const double* wts,
+                        int nd, int cplx, const Segs& sg, double* partial, double* out,
+                        cudaStream_t st) {
+  return launch_orth(V, ldv, m, const_cast<double*>(w), wts, nd, cplx, sg, partial, out, nullptr,
+                     0, nullptr, nullptr, st);
 }
 
 cudaError_t launch_dscale(const double* x, double* y, const double* s, int64_t n, int nd, int cplx,
@@ -2287,111 +2459,63 @@ cudaError_t launch_axpbys(const double* x, double* y, const double* a, double br
 }
 
 // ---- GMRES least squares on the device (FP64) -------------------------------
-// Complex values as (re, im) pairs; one thread per system.
-struct Z {
-  double r, i;
-};
-__device__ __forceinline__ Z zmul(Z a, Z b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
-__device__ __forceinline__ Z zadd(Z a, Z b) { return {a.r + b.r, a.i + b.i}; }
-__device__ __forceinline__ Z zconj(Z a) { return {a.r, -a.i}; }
-__device__ __forceinline__ Z zdiv(Z a, Z b) {
-  const double d = b.r * b.r + b.i * b.i;
-  return {(a.r * b.r + a.i * b.i) / d, (a.i * b.r - a.r * b.i) / d};
-}
-__device__ __forceinline__ Z zld(const double* p) { return {p[0], p[1]}; }
-__device__ __forceinline__ void zst(double* p, Z v) {
-  p[0] = v.r;
-  p[1] = v.i;
-}
-
-// Iteration it of every active system: the new Hessenberg column
-// H(0..it, it) = h1 + h2 (the two Gram-Schmidt passes) with zid on the
-// diagonal, the previous Givens rotations applied, the new rotation
-// (zrotmat_gmres, rotmat_gmres.f:60-100) against the norm of the new
-// vector, the rotated residual vector s, the residual estimate
-// |s(it+1)| / ||rhs||, and the stopping test; scale = 1/||w|| for the
-// systems that go on (0 for the others).  done[q]: 0 active, > 0 iterations
-// taken, < 0 zero right-hand side; brk[q] = 1 on a NaN (breakdown).
-__global__ void gmres_givens_kernel(int it, int M, int nsys, const double* __restrict__ h1,
-                                    const double* __restrict__ h2,
-                                    const double* __restrict__ nrm,
-                                    const double* __restrict__ zid, double* __restrict__ H,
-                                    double* __restrict__ cs, double* __restrict__ sn,
-                                    double* __restrict__ sv, const double* __restrict__ bnorm,
-                                    const double* __restrict__ eps, int64_t* __restrict__ done,
-                                    int* __restrict__ brk, double* __restrict__ errs,
-                                    double* __restrict__ scale) {
+// Start of a solve, one thread per system: from the squared norms of the
+// residual (nrm) and of the right-hand side (nrmb, null when there is no
+// initial guess): scale = 1/||r0||, s(0) = ||r0||, bnorm = ||rhs||, and
+// done = -1 for a zero residual (solution 0).
+__global__ void gmres_init_kernel(int M, int nsys, const double* __restrict__ nrm,
+                                  const double* __restrict__ nrmb, double* __restrict__ scale,
+                                  double* __restrict__ sv, double* __restrict__ bnorm,
+                                  int64_t* __restrict__ done, int* __restrict__ brk) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nsys) return;
-  scale[2 * q] = 0.0;
-  scale[2 * q + 1] = 0.0;
-  if (done[q] != 0) return;
-  double* Hq = H + 2 * (size_t(q) * M + it) * (M + 1);  // column it of system q
-  for (int k = 0; k <= it; ++k)
-    zst(Hq + 2 * k, zadd(zld(h1 + 2 * (size_t(k) * nsys + q)), zld(h2 + 2 * (size_t(k) * nsys + q))));
-  zst(Hq + 2 * it, zadd(zld(Hq + 2 * it), zld(zid + 2 * q)));
-  const double wnrm = sqrt(fmax(nrm[2 * q], 0.0));
-  double* cq = cs + 2 * size_t(q) * M;
-  double* sq = sn + 2 * size_t(q) * M;
-  double* vq = sv + 2 * size_t(q) * (M + 1);
-  for (int k = 0; k < it; ++k) {
-    const Z c = zld(cq + 2 * k), s = zld(sq + 2 * k);
-    const Z a = zld(Hq + 2 * k), b = zld(Hq + 2 * (k + 1));
-    zst(Hq + 2 * k, zadd(zmul(c, a), zmul(zconj(s), b)));
-    const Z ms = {-s.r, -s.i};
-    zst(Hq + 2 * (k + 1), zadd(zmul(ms, a), zmul(c, b)));
-  }
-  const Z a = zld(Hq + 2 * it);
-  Z c, s;
-  if (a.r == 0.0 && a.i == 0.0) {
-    c = {0.0, 0.0};
-    s = {1.0, 0.0};
-  } else {
-    const Z t = zdiv(Z{wnrm, 0.0}, a);
-    const double cr = 1.0 / sqrt(1.0 + t.r * t.r + t.i * t.i);
-    c = {cr, 0.0};
-    s = {t.r * cr, t.i * cr};
-  }
-  zst(cq + 2 * it, c);
-  zst(sq + 2 * it, s);
-  zst(Hq + 2 * it, zadd(zmul(c, a), zmul(zconj(s), Z{wnrm, 0.0})));
-  const Z v = zld(vq + 2 * it);
-  zst(vq + 2 * (it + 1), Z{-(s.r * v.r - s.i * v.i), -(s.r * v.i + s.i * v.r)});
-  zst(vq + 2 * it, zmul(c, v));
-  const Z vn = zld(vq + 2 * (it + 1));
-  const double err = bnorm[q] > 0.0 ? sqrt(vn.r * vn.r + vn.i * vn.i) / bnorm[q] : 0.0;
-  errs[size_t(q) * (M + 1) + it] = err;
-  if (!(err == err) || !(wnrm == wnrm)) {
-    brk[q] = 1;
-    done[q] = it + 1;
-    return;
-  }
-  // the new Krylov vector is normalised also when the system stops here: it
-  // is the last vector of the basis that carries the residual vector
-  if (wnrm > 0.0) scale[2 * q] = 1.0 / wnrm;
-  if (err <= eps[q] || it == M - 1 || wnrm == 0.0) done[q] = it + 1;
+  // (a NaN stays one: the first Givens step reports it)
+  auto root = [](double v) { return sqrt(v < 0.0 ? 0.0 : v); };
+  const double rb = root(nrm[2 * q]);
+  zst(scale + 2 * q, Z{rb > 0.0 ? 1.0 / rb : 0.0, 0.0});
+  zst(sv + 2 * size_t(q) * (M + 1), Z{rb, 0.0});
+  bnorm[q] = nrmb ? root(nrmb[2 * q]) : rb;
+  done[q] = rb == 0.0 ? -1 : 0;
+  brk[q] = 0;
+}
+
+cudaError_t launch_gmres_init(int M, int nsys, const double* nrm, const double* nrmb,
+                              double* scale, double* sv, double* bnorm, int64_t* done, int* brk,
+                              cudaStream_t st) {
+  gmres_init_kernel<<<(nsys + 63) / 64, 64, 0, st>>>(M, nsys, nrm, nrmb, scale, sv, bnorm, done,
+                                                     brk);
+  count();
+  return cudaGetLastError();
 }
 
 // y = triu(H)^-1 s over the done[q] iterations of system q, written as the
-// combination coefficients coef[2 (j nsys + q)], j < mused (zero past done[q]).
+// combination coefficients coef[2 (j nsys + q)], j < mused (zero past
+// done[q]).  One warp per system, by columns: lane l owns the entries j = l
+// (mod 32), so the only exchange is the new y_j.  (Row by row in one thread:
+// 67 us after 27 iterations.)
 __global__ void gmres_backsolve_kernel(int M, int nsys, int mused, const double* __restrict__ H,
                                        const double* __restrict__ sv,
                                        const int64_t* __restrict__ done,
                                        double* __restrict__ coef) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (q >= nsys) return;
   const int k = done[q] > 0 ? int(done[q]) : 0;
-  for (int j = k; j < mused; ++j) zst(coef + 2 * (size_t(j) * nsys + q), Z{0.0, 0.0});
-  const double* Hq = H + 2 * size_t(q) * M * (M + 1);
+  auto at = [&](int j) { return coef + 2 * (size_t(j) * nsys + q); };
   const double* vq = sv + 2 * size_t(q) * (M + 1);
+  for (int j = lane; j < mused; j += 32) zst(at(j), j < k ? zld(vq + 2 * j) : Z{0.0, 0.0});
+  const double* Hq = H + 2 * size_t(q) * M * (M + 1);
   for (int j = k - 1; j >= 0; --j) {
-    Z acc = zld(vq + 2 * j);
-    for (int l = j + 1; l < k; ++l) {
-      const Z h = zld(Hq + 2 * (size_t(l) * (M + 1) + j));
-      const Z y = zld(coef + 2 * (size_t(l) * nsys + q));
-      acc = {acc.r - (h.r * y.r - h.i * y.i), acc.i - (h.r * y.i + h.i * y.r)};
+    const double* col = Hq + 2 * size_t(j) * (M + 1);
+    Z y{0.0, 0.0};
+    if (lane == (j & 31)) {
+      y = zdiv(zld(at(j)), zld(col + 2 * j));
+      zst(at(j), y);
     }
-    zst(coef + 2 * (size_t(j) * nsys + q), zdiv(acc, zld(Hq + 2 * (size_t(j) * (M + 1) + j))));
+    y = zshfl(y, j & 31);
+    for (int l = lane; l < j; l += 32) {
+      const Z h = zld(col + 2 * l), v = zld(at(l));
+      zst(at(l), Z{v.r - (h.r * y.r - h.i * y.i), v.i - (h.r * y.i + h.i * y.r)});
+    }
   }
 }
 
@@ -2462,20 +2586,9 @@ cudaError_t launch_kx_update(double* kx, const double* r, const double* rn, cons
   return cudaGetLastError();
 }
 
-cudaError_t launch_gmres_givens(int it, int M, int nsys, const double* h1, const double* h2,
-                                const double* nrm, const double* zid, double* H, double* cs,
-                                double* sn, double* sv, const double* bnorm, const double* eps,
-                                int64_t* done, int* brk, double* errs, double* scale,
-                                cudaStream_t st) {
-  gmres_givens_kernel<<<(nsys + 63) / 64, 64, 0, st>>>(it, M, nsys, h1, h2, nrm, zid, H, cs, sn, sv,
-                                                       bnorm, eps, done, brk, errs, scale);
-  count();
-  return cudaGetLastError();
-}
-
 cudaError_t launch_gmres_backsolve(int M, int nsys, int mused, const double* H, const double* sv,
                                    const int64_t* done, double* coef, cudaStream_t st) {
-  gmres_backsolve_kernel<<<(nsys + 63) / 64, 64, 0, st>>>(M, nsys, mused, H, sv, done, coef);
+  gmres_backsolve_kernel<<<(nsys + 3) / 4, 128, 0, st>>>(M, nsys, mused, H, sv, done, coef);
   count();
   return cudaGetLastError();
 }

@@ -187,6 +187,7 @@ class Operator {
  private:
   DBuf<int64_t> chunk_lo_, chunk_hi_;
   DBuf<int32_t> seg_chunk0_, node_seg_;
+  DBuf<int> ticket_;
 };
 
 class Plan : public Operator {

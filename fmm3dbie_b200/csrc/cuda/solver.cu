@@ -68,6 +68,9 @@ int Operator::init_segments(cudaStream_t st) {
   segs.chunk_hi = chunk_hi_.p;
   segs.seg_chunk0 = seg_chunk0_.p;
   segs.node_seg = nullptr;
+  BIE_CUDA(ticket_.alloc(1));
+  BIE_CUDA(cudaMemsetAsync(ticket_.p, 0, sizeof(int), st));
+  segs.ticket = ticket_.p;
   if (ns > 1) {
     std::vector<int32_t> ns_of(nodes);
     for (int g = 0; g < ns; ++g)
@@ -101,16 +104,19 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
   BIE_CUDA(ws.partial.alloc(size_t(2) * (numit + 1) * nd * sg.nchunk));
   BIE_CUDA(ws.dots.alloc(size_t(2) * 3 * (numit + 1) * nsys));
   BIE_CUDA(ws.coef.alloc(size_t(2) * (numit + 1) * nsys));
-  BIE_CUDA(ws.scale.alloc(size_t(2) * 2 * nsys));
+  BIE_CUDA(ws.scale.alloc(size_t(5) * nsys));
   double* d_h1 = ws.dots.p;
   double* d_h2 = ws.dots.p + 2 * (numit + 1) * nsys;
   double* d_nrm = ws.dots.p + 4 * (numit + 1) * nsys;
   double* d_zid = ws.scale.p + 2 * nsys;  // zid per system
+  double* d_eps = ws.scale.p + 4 * nsys;  // stopping tolerance per system
   const double* wts = P.d_node_wts;
   double* V = ws.V.p;
-  std::vector<cdouble> zv(zid, zid + nsys);
+  std::vector<double> epsv(nsys);
   {
-    const std::vector<double> zh = interleave(zv);
+    std::vector<double> zh = interleave(std::vector<cdouble>(zid, zid + nsys));
+    for (int q = 0; q < nsys; ++q) epsv[q] = eps_sys ? eps_sys[q] : eps_gmres;
+    zh.insert(zh.end(), epsv.begin(), epsv.end());
     BIE_CUDA(cudaMemcpyAsync(d_zid, zh.data(), zh.size() * sizeof(double), cudaMemcpyHostToDevice, st));
   }
   // residual start: r0 = rhs - (zid x0 + K x0)  (stored in V_0 before scaling)
@@ -124,34 +130,17 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
     BIE_CUDA(cudaMemcpyAsync(V, d_rhs, ldv * sizeof(double), cudaMemcpyDeviceToDevice, st));
   }
   BIE_CUDA(dev::launch_mdot(V, ldv, 1, V, wts, nd, cplx, sg, ws.partial.p, d_nrm, st));
-  std::vector<double> hbuf(2 * nsys);
-  BIE_CUDA(cudaMemcpyAsync(hbuf.data(), d_nrm, 2 * nsys * sizeof(double), cudaMemcpyDeviceToHost, st));
-  BIE_CUDA(cudaStreamSynchronize(st));
-  std::vector<double> rb(nsys), bnorm(nsys);
-  std::vector<double> hscale(2 * nsys, 0.0);
-  for (int q = 0; q < nsys; ++q) {
-    rb[q] = std::sqrt(std::max(hbuf[2 * q], 0.0));
-    hscale[2 * q] = rb[q] > 0 ? 1.0 / rb[q] : 0.0;
-    bnorm[q] = rb[q];
-  }
   // With an initial guess the stopping test stays relative to ||rhs||_w, so a
   // warm-started solve meets the same accuracy as one from zero.
-  if (d_x0) {
-    BIE_CUDA(dev::launch_mdot(d_rhs, ldv, 1, d_rhs, wts, nd, cplx, sg, ws.partial.p, d_nrm, st));
-    std::vector<double> hb(2 * nsys);
-    BIE_CUDA(cudaMemcpyAsync(hb.data(), d_nrm, 2 * nsys * sizeof(double), cudaMemcpyDeviceToHost, st));
-    BIE_CUDA(cudaStreamSynchronize(st));
-    for (int q = 0; q < nsys; ++q) bnorm[q] = std::sqrt(std::max(hb[2 * q], 0.0));
-  }
-  BIE_CUDA(cudaMemcpyAsync(ws.scale.p, hscale.data(), 2 * nsys * sizeof(double), cudaMemcpyHostToDevice, st));
-  BIE_CUDA(dev::launch_dscale(V, V, ws.scale.p, n, nd, cplx, sg, st));
+  if (d_x0)
+    BIE_CUDA(dev::launch_mdot(d_rhs, ldv, 1, d_rhs, wts, nd, cplx, sg, ws.partial.p, d_h1, st));
   // Per-system Hessenberg columns, rotations and residual vector live on the
   // device; the Givens step and the back-substitution run there in FP64, and
   // the host reads back only the per-system stop flags each iteration.
   const int64_t M = numit;
   const size_t nH = size_t(2) * nsys * (M + 1) * M, nR = size_t(2) * nsys * M,
                nS = size_t(2) * nsys * (M + 1), nE = size_t(nsys) * (M + 1);
-  BIE_CUDA(ws.ls.alloc(nH + 2 * nR + nS + 2 * size_t(nsys) + nE));
+  BIE_CUDA(ws.ls.alloc(nH + 2 * nR + nS + size_t(nsys) + nE));
   BIE_CUDA(ws.done.alloc(nsys));
   BIE_CUDA(ws.brk.alloc(nsys));
   double* d_H = ws.ls.p;
@@ -159,25 +148,16 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
   double* d_sn = d_cs + nR;
   double* d_sv = d_sn + nR;
   double* d_bnorm = d_sv + nS;
-  double* d_eps = d_bnorm + nsys;
-  double* d_errs = d_eps + nsys;
-  std::vector<int64_t> done(nsys, 0);
-  std::vector<double> sv0(2 * nsys, 0.0), epsv(nsys);
-  int nactive = 0;
-  for (int q = 0; q < nsys; ++q) {
-    sv0[2 * q] = rb[q];
-    epsv[q] = eps_sys ? eps_sys[q] : eps_gmres;
-    if (rb[q] == 0.0) done[q] = -1;  // zero right-hand side: solution 0
-    else ++nactive;
-  }
-  // s(0) of system q = ||r0||; the rest of s is written as the rotations go
-  BIE_CUDA(cudaMemcpy2DAsync(d_sv, 2 * (M + 1) * sizeof(double), sv0.data(), 2 * sizeof(double),
-                             2 * sizeof(double), nsys, cudaMemcpyHostToDevice, st));
-  BIE_CUDA(cudaMemcpyAsync(d_bnorm, bnorm.data(), nsys * sizeof(double), cudaMemcpyHostToDevice, st));
-  BIE_CUDA(cudaMemcpyAsync(d_eps, epsv.data(), nsys * sizeof(double), cudaMemcpyHostToDevice, st));
-  BIE_CUDA(cudaMemcpyAsync(ws.done.p, done.data(), nsys * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+  double* d_errs = d_bnorm + nsys;
   BIE_CUDA(cudaMemsetAsync(d_errs, 0, nE * sizeof(double), st));
-  BIE_CUDA(cudaMemsetAsync(ws.brk.p, 0, nsys * sizeof(int), st));
+  BIE_CUDA(dev::launch_gmres_init(int(M), nsys, d_nrm, d_x0 ? d_h1 : nullptr, ws.scale.p, d_sv,
+                                  d_bnorm, ws.done.p, ws.brk.p, st));
+  BIE_CUDA(dev::launch_dscale(V, V, ws.scale.p, n, nd, cplx, sg, st));
+  std::vector<int64_t> done(nsys, 0);
+  BIE_CUDA(cudaMemcpyAsync(done.data(), ws.done.p, nsys * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  BIE_CUDA(cudaStreamSynchronize(st));
+  int nactive = 0;
+  for (int q = 0; q < nsys; ++q) nactive += done[q] == 0 ? 1 : 0;
   out.niter.assign(nsys, 0);
   out.errs.assign(nE, 0.0);
   out.rres.assign(nsys, 0.0);
@@ -196,14 +176,30 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
     ier = P.apply(precision, nd, vit, ws.w.p, st);
     if (ier) return ier;
     const int m = int(it + 1);
-    BIE_CUDA(dev::launch_mdot(V, ldv, m, ws.w.p, wts, nd, cplx, sg, ws.partial.p, d_h1, st));
-    BIE_CUDA(dev::launch_maxpy(V, ldv, m, d_h1, ws.w.p, n, nd, cplx, sg, st));
-    BIE_CUDA(dev::launch_mdot(V, ldv, m, ws.w.p, wts, nd, cplx, sg, ws.partial.p, d_h2, st));
-    BIE_CUDA(dev::launch_maxpy(V, ldv, m, d_h2, ws.w.p, n, nd, cplx, sg, st));
-    BIE_CUDA(dev::launch_mdot(ws.w.p, ldv, 1, ws.w.p, wts, nd, cplx, sg, ws.partial.p, d_nrm, st));
-    BIE_CUDA(dev::launch_gmres_givens(int(it), int(M), nsys, d_h1, d_h2, d_nrm, d_zid, d_H, d_cs,
-                                      d_sn, d_sv, d_bnorm, d_eps, ws.done.p, ws.brk.p, d_errs,
-                                      ws.scale.p, st));
+    // classical Gram-Schmidt twice, then the norm and the Givens step
+    dev::GivensArgs gv;
+    gv.it = int(it);
+    gv.M = int(M);
+    gv.nsys = nsys;
+    gv.h1 = d_h1;
+    gv.h2 = d_h2;
+    gv.nrm = d_nrm;
+    gv.zid = d_zid;
+    gv.H = d_H;
+    gv.cs = d_cs;
+    gv.sn = d_sn;
+    gv.sv = d_sv;
+    gv.bnorm = d_bnorm;
+    gv.eps = d_eps;
+    gv.done = ws.done.p;
+    gv.brk = ws.brk.p;
+    gv.errs = d_errs;
+    gv.scale = ws.scale.p;
+    double* w = ws.w.p;
+    double* pt = ws.partial.p;
+    BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h1, nullptr, 0, nullptr, nullptr, st));
+    BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h2, d_h1, m, V, nullptr, st));
+    BIE_CUDA(dev::launch_orth(w, ldv, 1, w, wts, nd, cplx, sg, pt, d_nrm, d_h2, m, V, &gv, st));
     BIE_CUDA(dev::launch_dscale(ws.w.p, vnext, ws.scale.p, n, nd, cplx, sg, st));
     BIE_CUDA(cudaMemcpyAsync(done.data(), ws.done.p, nsys * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     BIE_CUDA(cudaStreamSynchronize(st));
@@ -249,15 +245,11 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
     BIE_CUDA(dev::launch_axpby(d_rhs, ws.w.p, -1.0, 0.0, 1.0, 0.0, n, cplx, st));
     BIE_CUDA(dev::launch_mdot(ws.w.p, ldv, 1, ws.w.p, wts, nd, cplx, sg, ws.partial.p, d_nrm, st));
     BIE_CUDA(cudaMemcpyAsync(hn.data(), d_nrm, 2 * nsys * sizeof(double), cudaMemcpyDeviceToHost, st));
-    // ||rhs|| (the initial residual norm is ||rhs - A x0||, not ||rhs||)
-    BIE_CUDA(dev::launch_mdot(d_rhs, ldv, 1, d_rhs, wts, nd, cplx, sg, ws.partial.p, d_h1, st));
-    std::vector<double> hr(2 * nsys);
-    BIE_CUDA(cudaMemcpyAsync(hr.data(), d_h1, 2 * nsys * sizeof(double), cudaMemcpyDeviceToHost, st));
+    std::vector<double> bn(nsys);
+    BIE_CUDA(cudaMemcpyAsync(bn.data(), d_bnorm, nsys * sizeof(double), cudaMemcpyDeviceToHost, st));
     BIE_CUDA(cudaStreamSynchronize(st));
-    for (int q = 0; q < nsys; ++q) {
-      const double rn = std::sqrt(std::max(hr[2 * q], 0.0));
-      out.rres[q] = rn > 0 ? std::sqrt(std::max(hn[2 * q], 0.0)) / rn : 0.0;
-    }
+    for (int q = 0; q < nsys; ++q)
+      out.rres[q] = bn[q] > 0 ? std::sqrt(std::max(hn[2 * q], 0.0)) / bn[q] : 0.0;
   }
   return out.status;
 }
