@@ -1148,6 +1148,10 @@ int bie_plan_info(void* plan, int64_t* info) {
 
 int bie_plan_set_far(void* plan, int64_t iprec, int64_t nd, int64_t variant, int64_t nchunks) {
   if (!plan) return BIE_ERR_ARG;
+  if (variant > 4) {  // (5, the shape for few targets, is the autotuner's alone)
+    bie::set_last_error("far configuration out of range");
+    return BIE_ERR_ARG;
+  }
   return guarded([&] {
     return static_cast<bie::Plan*>(plan)->set_far_config(int(iprec), int(nd), int(variant),
                                                          int(nchunks));

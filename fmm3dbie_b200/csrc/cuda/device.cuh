@@ -127,6 +127,8 @@ int far_nchunks(int64_t ntarg, int64_t nptso, int kind, int precision, int nd, i
 // chunks that fills `waves` waves of resident blocks.
 // md = 1 selects the multi-density kernel's shapes (nd > 1).
 int far_variants();
+constexpr int kFarSmall = 5;  // one-density shape for few targets
+bool far_small_fits(int64_t ntarg, int nd);  // whether the autotuner tries it
 // Tensor-core far field (variants 3 and 4 of the multi-density FP32
 // Helmholtz path): densities per CTA, 0 where the variant does not apply.
 int far_tc_group(int variant, int nd, int precision, int kind);

@@ -22,6 +22,7 @@
 #include "device.cuh"
 
 #include "pair.cuh"
+#include "tile_eval.cuh"
 #include "trig_table.cuh"
 
 namespace bie {
@@ -405,6 +406,96 @@ __global__ void __launch_bounds__(NT, (kFarMinBlocks<R, NT>)) far_kernel(Geometr
     }
     far_block<KIND, R, NT, TPT, TILE, CK>(g, kp, str, partial, chunk_len, nd, blockIdx.x,
                                           blockIdx.y, blockIdx.z, tab, sg0, sg1, sst);
+  }
+}
+
+// Direct far field of small problems: one block per 32 targets and source
+// chunk, its four warps taking a quarter of every source tile each.  The
+// shapes above give a thread 1 to 8 targets and a whole tile, so a problem of
+// about a thousand targets leaves most of the chip without a warp and each
+// warp with a serial chain over 128 sources a tile.  864 targets x 2,646
+// sources (with about 5 us of launch and event time): Helmholtz FP64 21.6 ->
+// 15.8 us, FP32 17.4 -> 9.7, Laplace FP64 13.4 -> 11.1, FP32 13.0 -> 9.1; from
+// 5,400 targets on the other shapes are faster (they read each source for 2 to
+// 8 targets).  The target's sums of the four warps are added in order at the
+// end.
+constexpr int kSmallTargets = 32, kSmallThreads = 128;
+
+template <int KIND, typename R, bool CK>
+__global__ void __launch_bounds__(kSmallThreads)
+    far_small_kernel(Geometry g, KParams kp, const R* __restrict__ str,
+                     double* __restrict__ partial, int64_t chunk_len) {
+  using R4 = typename Vec<R>::T4;
+  constexpr int SW = KIND == 1 ? 4 : 2, TILE = kFarTileSources, PART = TILE / 4;
+  constexpr bool F32 = sizeof(R) == 4;
+  static_assert(TILE == kSmallThreads, "one source per thread");
+  __shared__ __align__(16) TileSmem<KIND, R, TILE> tile[2];
+  __shared__ double2 red[kSmallThreads];
+  __shared__ double2 stab[!F32 && KIND == 1 ? kFarTrigN : 1];
+  const double2* tab = nullptr;
+  if constexpr (!F32 && KIND == 1) {
+    fill_far_trig_table(stab);
+    tab = stab;
+  }
+  const int tid = threadIdx.x, part = tid >> 5, lane = tid & 31;
+  const int64_t it = int64_t(blockIdx.x) * kSmallTargets + lane;
+  const int64_t ic = it < g.ntarg ? it : g.ntarg - 1;
+  // FP32: centred like the other shapes, on the first target of the
+  // 512-target block
+  const int64_t t0 = it - lane;
+  const int64_t tb = t0 / kFarBlockTargets32;
+  const int64_t tc = tb * kFarBlockTargets32;
+  const double cx = F32 ? g.tx[tc] : 0.0, cy = F32 ? g.ty[tc] : 0.0, cz = F32 ? g.tz[tc] : 0.0;
+  const R tx = R(g.tx[ic] - cx), ty = R(g.ty[ic] - cy), tz = R(g.tz[ic] - cz);
+  const R thr2 = R(kp.thresh * kp.thresh), k = R(kp.kr), kim = R(kp.ki);
+  const int64_t s0 = int64_t(blockIdx.y) * chunk_len;
+  const int64_t s1 = min(s0 + chunk_len, g.nptso);
+  double accr = 0.0, acci = 0.0;
+  double rx = 0, ry = 0, rz = 0, rnx = 0, rny = 0, rnz = 0;
+  R4 rs{R(0), R(0), R(0), R(0)};
+  auto load = [&](int64_t sb) {  // past the chunk's end: its last source without strength
+    const int64_t s = min(sb + tid, s1 - 1);
+    rx = g.sx[s], ry = g.sy[s], rz = g.sz[s];
+    rnx = g.snx[s], rny = g.sny[s], rnz = g.snz[s];
+    rs = R4{R(0), R(0), R(0), R(0)};
+    if (sb + tid < s1) {
+      const R* sp = str + size_t(s) * SW;
+      rs.x = sp[0], rs.y = sp[1];
+      if constexpr (SW == 4) rs.z = sp[2], rs.w = sp[3];
+    }
+  };
+  if (s0 < s1) load(s0);
+  int b = 0;
+  for (int64_t sb = s0; sb < s1; sb += TILE, b ^= 1) {
+    auto& T = tile[b];
+    tile_store(T, tid, rx, ry, rz, rnx, rny, rnz, cx, cy, cz, rs);
+    if (sb + TILE < s1) load(sb + TILE);
+    __syncthreads();
+    R pr, pi;
+    if constexpr (F32)
+      tile_eval<KIND, CK, 0, TILE>(T, part * PART, (part + 1) * PART, tx, ty, tz, k, kim, thr2,
+                                   pr, pi);
+    else
+      tile_eval<KIND, CK, 0, TILE>(T, part * PART, (part + 1) * PART, tx, ty, tz, k, kim, thr2,
+                                   pr, pi, tab);
+    accr += double(pr);
+    acci += double(pi);
+  }
+  red[tid] = make_double2(accr, acci);
+  __syncthreads();
+  if (part != 0 || it >= g.ntarg) return;
+#pragma unroll
+  for (int p = 1; p < 4; ++p) {
+    const double2 v = red[lane + 32 * p];
+    accr += v.x;
+    acci += v.y;
+  }
+  const size_t o = size_t(blockIdx.y) * g.ntarg + it;
+  if (KIND == 1) {
+    partial[2 * o] = accr;
+    partial[2 * o + 1] = acci;
+  } else {
+    partial[o] = accr;
   }
 }
 
@@ -1775,10 +1866,32 @@ cudaError_t far_dispatch(const Geometry& g, const KParams& kp, const MatvecArgs&
   return launch_far_t<KIND, R, NT, TPT, CK>(g, kp, a, st);
 }
 
+// The autotuner tries the small-problem shape up to this many targets: at 2,400
+// it wins in FP32 (23.4 against 27.3 us, Helmholtz) and loses in FP64 (54
+// against 50), at 5,400 it loses everywhere.
+constexpr int64_t kSmallMax = 4096;
+
+template <int KIND, typename R, bool CK>
+cudaError_t far_small(const Geometry& g, const KParams& kp, const MatvecArgs& a, cudaStream_t st,
+                      int* occ) {
+  if (occ)
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, far_small_kernel<KIND, R, CK>,
+                                                         kSmallThreads, 0);
+  const int64_t tblocks = (g.ntarg + kSmallTargets - 1) / kSmallTargets;
+  int64_t chunk = (g.nptso + a.nchunks - 1) / a.nchunks;
+  chunk = ((chunk + kFarTile - 1) / kFarTile) * kFarTile;
+  far_small_kernel<KIND, R, CK>
+      <<<dim3(unsigned(tblocks), unsigned(a.nchunks)), kSmallThreads, 0, st>>>(
+          g, kp, static_cast<const R*>(a.strengths), a.partial, chunk);
+  return cudaGetLastError();
+}
+
 template <int KIND, typename R, bool CK>
 cudaError_t far_variant(int v, const Geometry& g, const KParams& kp, const MatvecArgs& a,
                         cudaStream_t st, int* occ) {
   switch (v) {
+    case kFarSmall:
+      return far_small<KIND, R, CK>(g, kp, a, st, occ);
     case 1:
       return far_dispatch<KIND, R, CK, 1>(g, kp, a, st, occ);
     case 2:
@@ -1878,7 +1991,7 @@ cudaError_t far_any(const Geometry& g, const KParams& kp, const MatvecArgs& a, c
                     int* occ) {
   const bool ck = kp.kind == 1 && kp.ki != 0.0;
   const int v = a.far_variant;
-  if (v >= 3 && occ) {  // the tensor-core shapes are multi-density only
+  if (v >= 3 && v != kFarSmall && occ) {  // the tensor-core shapes are multi-density only
     *occ = 0;
     return cudaSuccess;
   }
@@ -2234,10 +2347,13 @@ cudaError_t launch_source_consts(const Geometry& g, const KParams& kp, int preci
   return cudaGetLastError();
 }
 
-int far_variants() { return 5; }
+int far_variants() { return kFarSmall + 1; }
+
+bool far_small_fits(int64_t ntarg, int nd) { return nd == 1 && ntarg <= kSmallMax; }
 
 int far_block_targets(int precision, int variant, int md, int nd) {
   if (md && far_tc_group(variant, nd, precision, 1) > 0) return far_tc_targets();
+  if (!md && variant == kFarSmall) return kSmallTargets;
   const int v = variant < 0 || variant > 2 ? 0 : variant;
   if (md) return kMdShapes[md_class(nd)][v][0] * kMdShapes[md_class(nd)][v][1];
   return precision == 1 ? kF32Shapes[v][0] * kF32Shapes[v][1]

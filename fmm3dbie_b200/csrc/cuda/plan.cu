@@ -741,6 +741,7 @@ int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, F
     std::vector<FarConfig> cand;
     const int md = nd > 1;
     for (int v = 0; v < dev::far_variants(); ++v) {
+      if (v == dev::kFarSmall && !dev::far_small_fits(ntarg, nd)) continue;
       const int bps = dev::far_blocks_per_sm(kp, precision, v, md, nd);
       if (bps <= 0) continue;
       for (double waves : {1.0, 2.0, 4.0, 8.0}) {
@@ -768,12 +769,16 @@ int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, F
       a.far_variant = c.variant;
       a.nchunks = c.nchunks;
       BIE_CUDA(launch_far_stage(a, st));  // warm
+      // launches of tens of microseconds are timed four at a time: one alone
+      // is mostly event and launch latency
+      const int reps = double(ntarg) * double(nptso) * nd < 1e8 ? 4 : 1;
       BIE_CUDA(cudaEventRecord(e0, st));
-      BIE_CUDA(launch_far_stage(a, st));
+      for (int r = 0; r < reps; ++r) BIE_CUDA(launch_far_stage(a, st));
       BIE_CUDA(cudaEventRecord(e1, st));
       BIE_CUDA(cudaEventSynchronize(e1));
       float ms = 0;
       cudaEventElapsedTime(&ms, e0, e1);
+      ms /= reps;
       c.ms = ms;
       if (ms < best.ms) best = c;
       if (env_int("BIE_AUTOTUNE_LOG", 0))
