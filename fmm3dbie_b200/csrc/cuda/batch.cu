@@ -111,7 +111,7 @@ int BatchPlan::build_config(int precision, int nd, int variant, int64_t chunk, C
                             cudaStream_t st) {
   const int C = cplx ? 2 : 1;
   int tpb = 0, grp = 1;
-  dev::batch_far_shape(precision, variant, nd, &tpb, &grp);
+  dev::batch_far_shape(kind, precision, variant, nd, &tpb, &grp);
   const int groups = nd == 1 ? 1 : (nd + grp - 1) / grp;
   std::vector<dev::BatchSurf> hs(plans.size());
   std::vector<int2> patch_items, row_items;
@@ -209,7 +209,7 @@ int BatchPlan::tune(int precision, int nd, cudaStream_t st, std::unique_ptr<Conf
   std::vector<std::pair<int, int64_t>> cand;
   for (int v = 0; v < dev::batch_far_variants(precision, nd); ++v) {
     int tpb = 0, grp = 1;
-    dev::batch_far_shape(precision, v, nd, &tpb, &grp);
+    dev::batch_far_shape(kind, precision, v, nd, &tpb, &grp);
     const int groups = nd == 1 ? 1 : (nd + grp - 1) / grp;
     tot_blocks = 0;
     for (const auto& p : plans) tot_blocks += (p->ntarg + tpb - 1) / tpb * groups;

@@ -138,10 +138,10 @@ size_t far_tc_operand_floats(int nd, int precision, int kind, int64_t nptso);
 // Launches it, or with occ != null reports its resident CTAs per SM.
 cudaError_t far_tc(int variant, const Geometry& g, const KParams& kp, const MatvecArgs& a,
                    cudaStream_t st, int* occ);
-int far_block_targets(int precision, int variant, int md = 0, int nd = 1);
-int far_md_group(int variant, int nd);
+int far_block_targets(int kind, int precision, int variant, int md = 0, int nd = 1);
+int far_md_group(int kind, int precision, int variant, int nd);
 int far_blocks_per_sm(const KParams& kp, int precision, int variant, int md = 0, int nd = 1);
-int far_chunks_for_waves(int64_t ntarg, int64_t nptso, int precision, int variant, int nd,
+int far_chunks_for_waves(int kind, int64_t ntarg, int64_t nptso, int precision, int variant, int nd,
                          int num_sms, int blocks_per_sm, double waves, int md = 0);
 // Multi-density far field: a.strengths holds sigma_over[s][nd] (far
 // precision, from launch_oversample) and a.ab the per-source constants
@@ -282,7 +282,7 @@ struct BatchArgs {
 cudaError_t launch_batch_matvec(const BatchArgs& a, cudaStream_t st);
 // Far-kernel shape used by the batch: targets per block and densities per
 // block group for (precision, variant, nd); blocks per SM of the kernel.
-void batch_far_shape(int precision, int variant, int nd, int* targets_per_block, int* group);
+void batch_far_shape(int kind, int precision, int variant, int nd, int* targets_per_block, int* group);
 int batch_far_blocks_per_sm(int kind, int precision, int variant, int nd, bool ck);
 int batch_far_variants(int precision, int nd);
 

@@ -629,7 +629,7 @@ __device__ __forceinline__ void far_md_block(const Geometry& g, const KParams& k
           acc[t][m][C - 1] += double(tr2[t][m].y);
         }
     } else if constexpr (sizeof(R) == 4 && KIND == 0) {
-      // FP32 Laplace: two densities per packed multiply-add (fma.rn.f32x2,
+      // FP32 Laplace, 16 densities: two densities per packed multiply-add (fma.rn.f32x2,
       // each lane rounded as the scalar form).
       constexpr int NP = MD / 2;
       float2 tr2[TPT][NP];
@@ -735,25 +735,173 @@ __device__ __forceinline__ void far_md_block(const Geometry& g, const KParams& k
   }
 }
 
+// FP32 Laplace, several densities: two targets per packed instruction, the
+// source tile and its densities in shared memory with every value twice (the
+// layout of far_block_x2), tiles beyond the threshold margin without the
+// test.  The kernel value costs 12 packed operations and 2 rsqrt for two
+// pairs, a density one more; evaluated one target at a time the value took as
+// many instructions for each.
+// 36,504 nodes: 2.08 -> 1.70 ms at 4 densities, 2.56 -> 2.30 at 8; at 16 the
+// doubled densities' shared-memory reads make it 5 % slower (4.48 against
+// 4.25), so those blocks stay with far_md_block.
+template <int KIND, typename R, int MD>
+constexpr bool kMdLap32 = KIND == 0 && sizeof(R) == 4 && MD <= 8;
+template <int MD>
+constexpr int kMdLapWords = 4 + MD / 2;  // float4 per source
+
+template <int NT, int TPT, int MD, int TILE>
+__device__ __forceinline__ void far_md_lap_block(const Geometry& g, const KParams& kp,
+                                                 const float* __restrict__ ab,
+                                                 const float* __restrict__ sig, int nd,
+                                                 double* __restrict__ partial, int64_t chunk_len,
+                                                 int64_t bx, int64_t by, int bz, float4* tile) {
+  static_assert(TPT % 2 == 0 && kMdCentre % (NT * TPT) == 0, "target pairs, one centre");
+  constexpr int TP = TPT / 2, W = kMdLapWords<MD>;
+  const int64_t ntarg = g.ntarg, nptso = g.nptso;
+  const int64_t tbase = int64_t(bx) * NT * TPT;
+  const int m0 = bz * MD;
+  const int64_t tcen = (tbase / kMdCentre) * kMdCentre;
+  const int64_t tc = tcen < ntarg ? tcen : ntarg - 1;
+  const double cx = g.tx[tc], cy = g.ty[tc], cz = g.tz[tc];
+  float2 tx[TP], ty[TP], tz[TP];
+  double acc[TPT][MD];
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) {
+    const int64_t it = tbase + threadIdx.x + int64_t(t) * NT;
+    const int64_t ic = it < ntarg ? it : ntarg - 1;
+    const float x = float(g.tx[ic] - cx), y = float(g.ty[ic] - cy), z = float(g.tz[ic] - cz);
+    if (t % 2 == 0)
+      tx[t / 2].x = x, ty[t / 2].x = y, tz[t / 2].x = z;
+    else
+      tx[t / 2].y = x, ty[t / 2].y = y, tz[t / 2].y = z;
+#pragma unroll
+    for (int m = 0; m < MD; ++m) acc[t][m] = 0.0;
+  }
+  const float thr2 = float(kp.thresh * kp.thresh);
+  double tbx[6] = {0, 0, 0, 0, 0, 0};
+  const bool boxes = g.sbox && g.tbox && TILE == kFarTileSources && kMdCentre == kFarBlockTargets32;
+  if (boxes)
+#pragma unroll
+    for (int c = 0; c < 6; ++c) tbx[c] = g.tbox[6 * (tbase / kFarBlockTargets32) + c];
+  const int64_t s0 = int64_t(by) * chunk_len;
+  const int64_t s1 = min(s0 + chunk_len, nptso);
+  for (int64_t sb = s0; sb < s1; sb += TILE) {
+    const int ns = int((s1 - sb) < TILE ? (s1 - sb) : TILE);
+    __syncthreads();
+    for (int q = threadIdx.x; q < TILE; q += NT) {
+      float4* T = tile + q * W;
+      if (q < ns) {
+        const int64_t s = sb + q;
+        const float x = -float(g.sx[s] - cx), y = -float(g.sy[s] - cy), z = -float(g.sz[s] - cz);
+        const float nx = float(g.snx[s]), ny = float(g.sny[s]), nz = float(g.snz[s]);
+        const float2 v = reinterpret_cast<const float2*>(ab)[s];
+        T[0] = make_float4(x, x, y, y);
+        T[1] = make_float4(z, z, nx, nx);
+        T[2] = make_float4(ny, ny, nz, nz);
+        T[3] = make_float4(v.x, v.x, v.y, v.y);
+      } else {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) T[w] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+    for (int q = threadIdx.x; q < TILE * (MD / 2); q += NT) {
+      const int qs = q / (MD / 2), mm = 2 * (q - qs * (MD / 2));
+      const float* p = sig + size_t(sb + qs) * nd + m0 + mm;
+      const float a = qs < ns && m0 + mm < nd ? p[0] : 0.f;
+      const float b = qs < ns && m0 + mm + 1 < nd ? p[1] : 0.f;
+      tile[qs * W + 4 + mm / 2] = make_float4(a, a, b, b);
+    }
+    __syncthreads();
+    float2 tr[TP][MD];
+#pragma unroll
+    for (int t = 0; t < TP; ++t)
+#pragma unroll
+      for (int m = 0; m < MD; ++m) tr[t][m] = make_float2(0.f, 0.f);
+    bool check = true;
+    if (boxes && ns == TILE) {
+      const double* sbx = g.sbox + 6 * (sb / kFarTileSources);
+      double gap2 = 0.0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const double gap = fmax(fmax(sbx[c] - tbx[c + 3], tbx[c] - sbx[c + 3]), 0.0);
+        gap2 += gap * gap;
+      }
+      check = gap2 <= g.box_margin2;
+    }
+    auto sweep = [&](auto chk) {
+      constexpr bool C = decltype(chk)::value;
+#pragma unroll 2
+      for (int j = 0; j < TILE; ++j) {
+        const float4* T = tile + j * W;
+        const float4 q0 = T[0], q1 = T[1], q2 = T[2], q3 = T[3];
+        const float2 msx = make_float2(q0.x, q0.y), msy = make_float2(q0.z, q0.w),
+                     msz = make_float2(q1.x, q1.y), nx = make_float2(q1.z, q1.w),
+                     ny = make_float2(q2.x, q2.y), nz = make_float2(q2.z, q2.w),
+                     c = make_float2(q3.x, q3.y), d = make_float2(q3.z, q3.w);
+        float2 kv[TP];
+#pragma unroll
+        for (int t = 0; t < TP; ++t) {
+          kv[t] = make_float2(0.f, 0.f);
+          pair_lap_x2<C>(tx[t], ty[t], tz[t], msx, msy, msz, nx, ny, nz, c, d, thr2, kv[t]);
+        }
+#pragma unroll
+        for (int m = 0; m < MD; m += 2) {
+          const float4 x = T[4 + m / 2];
+#pragma unroll
+          for (int t = 0; t < TP; ++t) {
+            tr[t][m] = __ffma2_rn(kv[t], make_float2(x.x, x.y), tr[t][m]);
+            tr[t][m + 1] = __ffma2_rn(kv[t], make_float2(x.z, x.w), tr[t][m + 1]);
+          }
+        }
+      }
+    };
+    if (check)
+      sweep(std::true_type{});
+    else
+      sweep(std::false_type{});
+#pragma unroll
+    for (int t = 0; t < TP; ++t)
+#pragma unroll
+      for (int m = 0; m < MD; ++m) {
+        acc[2 * t][m] += double(tr[t][m].x);
+        acc[2 * t + 1][m] += double(tr[t][m].y);
+      }
+  }
+#pragma unroll
+  for (int t = 0; t < TPT; ++t) {
+    const int64_t it = tbase + threadIdx.x + int64_t(t) * NT;
+    if (it >= ntarg) continue;
+#pragma unroll
+    for (int m = 0; m < MD; ++m)
+      if (m0 + m < nd) partial[(size_t(by) * ntarg + it) * nd + m0 + m] = acc[t][m];
+  }
+}
+
 template <int KIND, typename R, int NT, int TPT, int MD, int TILE, bool CK>
 __global__ void __launch_bounds__(NT) far_md_kernel(Geometry g, KParams kp,
                                                     const R* __restrict__ ab,
                                                     const R* __restrict__ sig, int nd,
                                                     double* __restrict__ partial,
                                                     int64_t chunk_len) {
-  constexpr int C = (KIND == 1) ? 2 : 1;
-  __shared__ typename Vec<R>::T4 sg0[TILE];
-  __shared__ typename Vec<R>::T2 sg1[TILE];
-  __shared__ __align__(16) R sab[TILE * 2 * C];
-  __shared__ __align__(16) R ssig[TILE * MD * kMdSigWords<KIND, R, MD>];
-  __shared__ double2 stab[sizeof(R) == 8 && KIND == 1 ? kFarTrigN : 1];
-  const double2* tab = nullptr;
-  if constexpr (sizeof(R) == 8 && KIND == 1) {
-    fill_far_trig_table(stab);
-    tab = stab;
+  if constexpr (kMdLap32<KIND, R, MD>) {
+    __shared__ float4 tile[TILE * kMdLapWords<MD>];
+    far_md_lap_block<NT, TPT, MD, TILE>(g, kp, ab, sig, nd, partial, chunk_len, blockIdx.x,
+                                        blockIdx.y, blockIdx.z, tile);
+  } else {
+    constexpr int C = (KIND == 1) ? 2 : 1;
+    __shared__ typename Vec<R>::T4 sg0[TILE];
+    __shared__ typename Vec<R>::T2 sg1[TILE];
+    __shared__ __align__(16) R sab[TILE * 2 * C];
+    __shared__ __align__(16) R ssig[TILE * MD * kMdSigWords<KIND, R, MD>];
+    __shared__ double2 stab[sizeof(R) == 8 && KIND == 1 ? kFarTrigN : 1];
+    const double2* tab = nullptr;
+    if constexpr (sizeof(R) == 8 && KIND == 1) {
+      fill_far_trig_table(stab);
+      tab = stab;
+    }
+    far_md_block<KIND, R, NT, TPT, MD, TILE, CK>(g, kp, ab, sig, nd, partial, chunk_len, blockIdx.x,
+                                                 blockIdx.y, blockIdx.z, tab, sg0, sg1, sab, ssig);
   }
-  far_md_block<KIND, R, NT, TPT, MD, TILE, CK>(g, kp, ab, sig, nd, partial, chunk_len, blockIdx.x,
-                                               blockIdx.y, blockIdx.z, tab, sg0, sg1, sab, ssig);
 }
 
 // sigma_over[s][m] = (imat sigma_patch)[s][m] without scaling (several
@@ -1914,12 +2062,19 @@ constexpr int kMdShapes[3][3][3] = {
 template <typename R, int MD>
 constexpr int kMdTile = sizeof(R) == 8 && MD == 16 ? kFarTile / 2 : kFarTile;
 
+// Targets per thread: twice the table's for FP32 Laplace blocks of up to 8
+// densities, which take targets in pairs (far_md_lap_block).
+constexpr int md_tpt(int kind, int precision, int cl, int v) {
+  return kMdShapes[cl][v][1] * (kind == 0 && precision == 1 && cl < 2 ? 2 : 1);
+}
+
 inline int md_class(int nd) { return nd <= 4 ? 0 : (nd <= 8 ? 1 : 2); }
 
 template <int KIND, typename R, bool CK, int CL, int V>
 cudaError_t far_md_dispatch(const Geometry& g, const KParams& kp, const MatvecArgs& a,
                             cudaStream_t st, int* occ) {
-  constexpr int NT = kMdShapes[CL][V][0], TPT = kMdShapes[CL][V][1], MD = kMdShapes[CL][V][2];
+  constexpr int NT = kMdShapes[CL][V][0], TPT = md_tpt(KIND, sizeof(R) == 4, CL, V),
+                MD = kMdShapes[CL][V][2];
   if (occ) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         occ, far_md_kernel<KIND, R, NT, TPT, MD, kMdTile<R, MD>, CK>, NT, 0);
@@ -2089,10 +2244,12 @@ __global__ void __launch_bounds__(NT)
                         int nitems, const R* __restrict__ sig, double* __restrict__ partial,
                         int nd, int prec, int* __restrict__ counter) {
   constexpr int C = (KIND == 1) ? 2 : 1;
-  __shared__ typename Vec<R>::T4 sg0[TILE];
-  __shared__ typename Vec<R>::T2 sg1[TILE];
-  __shared__ __align__(16) R sab[TILE * 2 * C];
-  __shared__ __align__(16) R ssig[TILE * MD * kMdSigWords<KIND, R, MD>];
+  constexpr bool LAP32 = kMdLap32<KIND, R, MD>;
+  __shared__ float4 tile[LAP32 ? TILE * kMdLapWords<MD> : 1];
+  __shared__ typename Vec<R>::T4 sg0[LAP32 ? 1 : TILE];
+  __shared__ typename Vec<R>::T2 sg1[LAP32 ? 1 : TILE];
+  __shared__ __align__(16) R sab[LAP32 ? 4 : TILE * 2 * C];
+  __shared__ __align__(16) R ssig[LAP32 ? 4 : TILE * MD * kMdSigWords<KIND, R, MD>];
   __shared__ double2 stab[sizeof(R) == 8 && KIND == 1 ? kFarTrigN : 1];
   const double2* tab = nullptr;
   if constexpr (sizeof(R) == 8 && KIND == 1) {
@@ -2109,9 +2266,14 @@ __global__ void __launch_bounds__(NT)
     if (S.live && *S.live == 0) continue;  // uniform over the block
     const Geometry g = S.g;
     const KParams kp = S.kp;
-    far_md_block<KIND, R, NT, TPT, MD, TILE, CK>(
-        g, kp, static_cast<const R*>(S.ab[prec]), sig + S.sofs * nd * C, nd,
-        partial + S.pofs[prec], S.chunk_len[prec], it.y, it.z, it.w, tab, sg0, sg1, sab, ssig);
+    if constexpr (LAP32)
+      far_md_lap_block<NT, TPT, MD, TILE>(g, kp, static_cast<const R*>(S.ab[prec]),
+                                          sig + S.sofs * nd, nd, partial + S.pofs[prec],
+                                          S.chunk_len[prec], it.y, it.z, it.w, tile);
+    else
+      far_md_block<KIND, R, NT, TPT, MD, TILE, CK>(
+          g, kp, static_cast<const R*>(S.ab[prec]), sig + S.sofs * nd * C, nd,
+          partial + S.pofs[prec], S.chunk_len[prec], it.y, it.z, it.w, tab, sg0, sg1, sab, ssig);
     __syncthreads();
   }
 }
@@ -2161,7 +2323,8 @@ cudaError_t batch_far_dispatch(const BatchArgs& a, cudaStream_t st, int* occ) {
 
 template <int KIND, typename R, bool CK, int CL, int V>
 cudaError_t batch_far_md_dispatch(const BatchArgs& a, cudaStream_t st, int* occ) {
-  constexpr int NT = kMdShapes[CL][V][0], TPT = kMdShapes[CL][V][1], MD = kMdShapes[CL][V][2];
+  constexpr int NT = kMdShapes[CL][V][0], TPT = md_tpt(KIND, sizeof(R) == 4, CL, V),
+                MD = kMdShapes[CL][V][2];
   auto kern = batch_far_md_kernel<KIND, R, NT, TPT, MD, kMdTile<R, MD>, CK>;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, NT, 0);
   kern<<<a.grid_far, NT, 0, st>>>(a.surfs, a.far_items, a.nfar_items,
@@ -2203,7 +2366,8 @@ cudaError_t batch_far_any(const BatchArgs& a, cudaStream_t st, int* occ) {
 }
 }  // namespace
 
-void batch_far_shape(int precision, int variant, int nd, int* targets_per_block, int* group) {
+void batch_far_shape(int kind, int precision, int variant, int nd, int* targets_per_block,
+                     int* group) {
   const int v = variant < 0 || variant > 2 ? 0 : variant;
   if (nd == 1) {
     const int(*sh)[2] = precision == 1 ? kF32Shapes : kF64Shapes;
@@ -2212,7 +2376,7 @@ void batch_far_shape(int precision, int variant, int nd, int* targets_per_block,
     return;
   }
   const int cl = md_class(nd);
-  *targets_per_block = kMdShapes[cl][v][0] * kMdShapes[cl][v][1];
+  *targets_per_block = kMdShapes[cl][v][0] * md_tpt(kind, precision, cl, v);
   *group = kMdShapes[cl][v][2];
 }
 
@@ -2351,17 +2515,17 @@ int far_variants() { return kFarSmall + 1; }
 
 bool far_small_fits(int64_t ntarg, int nd) { return nd == 1 && ntarg <= kSmallMax; }
 
-int far_block_targets(int precision, int variant, int md, int nd) {
-  if (md && far_tc_group(variant, nd, precision, 1) > 0) return far_tc_targets();
+int far_block_targets(int kind, int precision, int variant, int md, int nd) {
+  if (md && far_tc_group(variant, nd, precision, kind) > 0) return far_tc_targets();
   if (!md && variant == kFarSmall) return kSmallTargets;
   const int v = variant < 0 || variant > 2 ? 0 : variant;
-  if (md) return kMdShapes[md_class(nd)][v][0] * kMdShapes[md_class(nd)][v][1];
+  if (md) return kMdShapes[md_class(nd)][v][0] * md_tpt(kind, precision, md_class(nd), v);
   return precision == 1 ? kF32Shapes[v][0] * kF32Shapes[v][1]
                         : kF64Shapes[v][0] * kF64Shapes[v][1];
 }
 
-int far_md_group(int variant, int nd) {
-  const int tc = far_tc_group(variant, nd, 1, 1);
+int far_md_group(int kind, int precision, int variant, int nd) {
+  const int tc = far_tc_group(variant, nd, precision, kind);
   if (tc > 0) return tc;
   return kMdShapes[md_class(nd)][variant < 0 || variant > 2 ? 0 : variant][2];
 }
@@ -2380,11 +2544,13 @@ int far_blocks_per_sm(const KParams& kp, int precision, int variant, int md, int
   return occ;
 }
 
-int far_chunks_for_waves(int64_t ntarg, int64_t nptso, int precision, int variant, int nd,
+int far_chunks_for_waves(int kind, int64_t ntarg, int64_t nptso, int precision, int variant, int nd,
                          int num_sms, int blocks_per_sm, double waves, int md) {
-  const int64_t bt = far_block_targets(precision, variant, md, nd);
+  const int64_t bt = far_block_targets(kind, precision, variant, md, nd);
   const int64_t tblocks = (ntarg + bt - 1) / bt;
-  const int64_t zdim = md ? (nd + far_md_group(variant, nd) - 1) / far_md_group(variant, nd) : nd;
+  const int64_t zdim = md ? (nd + far_md_group(kind, precision, variant, nd) - 1) /
+                                far_md_group(kind, precision, variant, nd)
+                          : nd;
   const double slots = double(num_sms) * std::max(blocks_per_sm, 1) * waves;
   int64_t s = std::max<int64_t>(1, int64_t(slots / double(tblocks * zdim) + 0.5));
   s = std::min<int64_t>(s, std::max<int64_t>(1, (nptso + kFarTile - 1) / kFarTile));

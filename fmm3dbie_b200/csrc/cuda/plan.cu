@@ -706,7 +706,7 @@ Plan::FarConfig Plan::far_config(int precision, int nd) const {
   const int md = nd > 1;
   c.variant = std::min(std::max(env_int("BIE_FAR_VARIANT", 0), 0), dev::far_variants() - 1);
   const int bps = dev::far_blocks_per_sm(kp, precision, c.variant, md, nd);
-  c.nchunks = dev::far_chunks_for_waves(ntarg, nptso, precision, c.variant, nd, num_sms, bps,
+  c.nchunks = dev::far_chunks_for_waves(kind, ntarg, nptso, precision, c.variant, nd, num_sms, bps,
                                         env_double("BIE_FAR_WAVES", md ? 2.0 : 4.0), md);
   return c;
 }
@@ -748,7 +748,7 @@ int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, F
         FarConfig c;
         c.variant = v;
         c.nchunks =
-            dev::far_chunks_for_waves(ntarg, nptso, precision, v, nd, num_sms, bps, waves, md);
+            dev::far_chunks_for_waves(kind, ntarg, nptso, precision, v, nd, num_sms, bps, waves, md);
         // the partial sums grow with nchunks * nd: keep them under ~1 GiB
         if (double(c.nchunks) * ntarg * nd * 16.0 > double(1 << 30) && waves > 1.0) continue;
         bool dup = false;
