@@ -97,12 +97,22 @@ struct Stage {
   }
 };
 
+// Uninitialised host array (the near quadrature is written whole; a vector
+// would first fill its pages with zeros on one thread).
+struct HostBuf {
+  std::unique_ptr<double[]> p;
+  void alloc(size_t n) { p.reset(new double[n > 0 ? n : 1]); }
+  double* data() { return p.get(); }
+  double& operator[](size_t i) { return p[i]; }
+};
+
 // Everything the simple interfaces derive from the geometry (the setup part
 // of lap_comb_dir_eval / helm_comb_dir_solver).
 struct Setup {
   std::vector<double> cms, rads;
   std::vector<int64_t> row_ptr, col_ind, iquad, novers, ixyzso;
-  std::vector<double> srcover, wover, wnear;
+  std::vector<double> srcover, wover;
+  HostBuf wnear;
   int64_t nnz = 0, nquad = 0, nptso = 0;
   double rfac = 0, rfac0 = 0;
 };
@@ -183,7 +193,7 @@ int run_setup(const bie::Surf& s, int kind, cdouble zk, cdouble alpha, cdouble b
                            nullptr, o.srcover.data());
   bie::qwts(so, o.wover.data());
   const size_t wl = size_t(o.nquad) * (kind == 1 ? 2 : 1);
-  o.wnear.assign(wl, 0.0);
+  o.wnear.alloc(wl);
   if (on_device && o.nnz > 0) {
     bie::DBuf<double> d_w;
     if (d_w.alloc(wl) != cudaSuccess) {
@@ -192,11 +202,10 @@ int run_setup(const bie::Surf& s, int kind, cdouble zk, cdouble alpha, cdouble b
     }
     ier = bie::getnearquad_gpu(s, ndtarg, ntarg, targs, ipatch_id, uvs_targ, eps, kind, zk, alpha,
                                beta, o.nnz, o.row_ptr.data(), o.col_ind.data(), o.iquad.data(),
-                               o.nquad, d_w.p, stg->st);
+                               o.nquad, d_w.p, stg->st, nullptr,
+                               [&] { bie::prefault(o.wnear.data(), wl * sizeof(double)); });
     if (ier) return ier;
-    if (cudaMemcpyAsync(o.wnear.data(), d_w.p, wl * sizeof(double), cudaMemcpyDeviceToHost,
-                        stg->st) != cudaSuccess ||
-        cudaStreamSynchronize(stg->st) != cudaSuccess) {
+    if (bie::copy_to_host(o.wnear.data(), d_w.p, wl * sizeof(double), stg->st) != cudaSuccess) {
       bie::set_last_error("near quadrature: copy to host failed");
       return BIE_ERR_CUDA;
     }
@@ -713,11 +722,10 @@ int nearquad_gpu_call(int kind, cdouble zk, cdouble alpha, cdouble beta, int64_t
   bie::NearQuadStats st;
   ier = bie::getnearquad_gpu(make_surf(npatches, norders, ixyzs, iptype, npts, srccoefs, srcvals),
                              int(ndtarg), ntarg, targs, ipatch_id, uvs_targ, eps, kind, zk, alpha,
-                             beta, nnz, row_ptr, col_ind, iquad, nquad, d_w.p, stg.st, &st);
+                             beta, nnz, row_ptr, col_ind, iquad, nquad, d_w.p, stg.st, &st,
+                             [&] { bie::prefault(wnear, wl * sizeof(double)); });
   if (ier) return ier;
-  if (wl && (cudaMemcpyAsync(wnear, d_w.p, wl * sizeof(double), cudaMemcpyDeviceToHost,
-                             stg.st) != cudaSuccess ||
-             cudaStreamSynchronize(stg.st) != cudaSuccess)) {
+  if (wl && bie::copy_to_host(wnear, d_w.p, wl * sizeof(double), stg.st) != cudaSuccess) {
     bie::set_last_error("getnearquad: copy to host failed");
     return BIE_ERR_CUDA;
   }

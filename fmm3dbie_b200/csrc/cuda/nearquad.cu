@@ -617,7 +617,8 @@ int getnearquad_gpu(const Surf& s, int ndt, int64_t nt, const double* targs,
                     const int64_t* ipatch_id, const double* uvs_targ, double eps, int kind,
                     cdouble zk, cdouble alpha, cdouble beta, int64_t nnz, const int64_t* row_ptr,
                     const int64_t* col_ind, const int64_t* iquad, int64_t nquad,
-                    double* wnear_dev, cudaStream_t st, NearQuadStats* stats) {
+                    double* wnear_dev, cudaStream_t st, NearQuadStats* stats,
+                    const std::function<void()>& while_running) {
   if (stats) *stats = NearQuadStats{};
   if (nnz == 0) return kOk;
   if (nnz < 0 || nt <= 0 || ndt < 3 || !targs || !row_ptr || !col_ind || !iquad || !wnear_dev ||
@@ -898,6 +899,7 @@ int getnearquad_gpu(const Surf& s, int ndt, int64_t nt, const double* targs,
   }
   cudaEventRecord(ev[1], st);
   dev::note_launches(launches);
+  if (while_running) while_running();
   unsigned long long cnt[2] = {0, 0};
   cudaMemcpyAsync(cnt, d_cnt.p + nlaunch, sizeof cnt, cudaMemcpyDeviceToHost, st);
   e = cudaStreamSynchronize(st);

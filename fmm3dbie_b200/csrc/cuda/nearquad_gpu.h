@@ -14,6 +14,7 @@
 // threshold and summation order can differ).
 #pragma once
 #include <cstdint>
+#include <functional>
 
 #include <cuda_runtime.h>
 
@@ -28,13 +29,15 @@ constexpr int kNearQuadMaxNp = 256;
 // Inputs are host arrays in the reference layout (1-based index arrays);
 // wnear_dev is device memory: nquad reals (kind 0) or nquad interleaved
 // complex values (kind 1).  Work runs on `st`; the call returns after the
-// stream has finished.  Returns kOk, kErrArg (inconsistent input or a patch
+// stream has finished; while_running (if given) runs on the calling thread
+// once everything is launched.  Returns kOk, kErrArg (inconsistent input or a patch
 // with more than kNearQuadMaxNp basis functions), kErrCuda, or kErrTimeout
 // when a pair hit the refinement-step cap.
 int getnearquad_gpu(const Surf& s, int ndt, int64_t nt, const double* targs,
                     const int64_t* ipatch_id, const double* uvs_targ, double eps, int kind,
                     cdouble zk, cdouble alpha, cdouble beta, int64_t nnz, const int64_t* row_ptr,
                     const int64_t* col_ind, const int64_t* iquad, int64_t nquad,
-                    double* wnear_dev, cudaStream_t st, NearQuadStats* stats = nullptr);
+                    double* wnear_dev, cudaStream_t st, NearQuadStats* stats = nullptr,
+                    const std::function<void()>& while_running = {});
 
 }  // namespace bie

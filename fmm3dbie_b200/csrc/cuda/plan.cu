@@ -110,6 +110,7 @@ class HostStaging {
   }
   HostStaging(const HostStaging&) = delete;
   HostStaging& operator=(const HostStaging&) = delete;
+  bool pinned() const { return !heap_; }
   // the stream that the uploads out of the buffer are issued on
   void copies_on(cudaStream_t st) {
     st_ = st;
@@ -141,6 +142,67 @@ class HostStaging {
   std::unique_ptr<char[]> heap_;
 };
 }  // namespace
+
+void prefault(void* p, size_t bytes) {
+  constexpr size_t page = 4096;
+  char* c = static_cast<char*>(p);
+  const int64_t n = int64_t((bytes + page - 1) / page);
+#pragma omp parallel for schedule(static) if (n >= 256)
+  for (int64_t q = 0; q < n; ++q) {
+    volatile char* v = c + size_t(q) * page;
+    *v = *v;
+  }
+}
+
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  constexpr size_t piece = size_t(4) << 20;
+  constexpr int slots = 4;
+  cudaPointerAttributes at{};
+  const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+                      at.type != cudaMemoryTypeUnregistered;
+  if (!pinned) cudaGetLastError();
+  if (pinned || bytes < 2 * piece) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+  }
+  HostStaging stage(slots * piece);
+  if (!stage.pinned()) {  // in use by another thread
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+  }
+  stage.copies_on(st);
+  char* slot[slots];
+  cudaEvent_t ev[slots] = {};
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < slots; ++i) {
+    slot[i] = stage.take<char>(piece);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+  }
+  const size_t np = (bytes + piece - 1) / piece;
+  auto len = [&](size_t q) { return std::min(piece, bytes - q * piece); };
+  auto issue = [&](size_t q) {
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(slot[q % slots], static_cast<const char*>(src) + q * piece, len(q),
+                          cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaEventRecord(ev[q % slots], st);
+  };
+  for (size_t q = 0; q < std::min<size_t>(slots, np); ++q) issue(q);
+  for (size_t q = 0; q < np && e == cudaSuccess; ++q) {
+    e = cudaEventSynchronize(ev[q % slots]);
+    if (e != cudaSuccess) break;
+    const char* from = slot[q % slots];
+    char* to = static_cast<char*>(dst) + q * piece;
+    const size_t n = len(q);
+    constexpr size_t part = size_t(256) << 10;
+#pragma omp parallel for schedule(static)
+    for (size_t o = 0; o < n; o += part) std::memcpy(to + o, from + o, std::min(part, n - o));
+    if (q + slots < np) issue(q + slots);
+  }
+  const cudaError_t es = cudaStreamSynchronize(st);
+  for (auto& v : ev)
+    if (v) cudaEventDestroy(v);
+  return e != cudaSuccess ? e : es;
+}
 
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 const char* last_error() { return g_last_error.c_str(); }

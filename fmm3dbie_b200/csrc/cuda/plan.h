@@ -58,6 +58,16 @@ struct AllocStreamScope {
   AllocStreamScope& operator=(const AllocStreamScope&) = delete;
 };
 
+// Touches every page of a host buffer that a running device computation will
+// fill, with several threads and without changing its contents: the pages of
+// a fresh allocation are then in place when the result arrives.
+void prefault(void* p, size_t bytes);
+// Copies device memory to a host buffer and waits for it.  Pageable buffers of
+// several MB go through the process's pinned staging buffer in pieces that
+// several threads move on while the next ones arrive (the driver's own
+// pageable copy: about 5 GB/s into fresh pages).
+cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
+
 template <class T>
 struct DBuf {
   T* p = nullptr;
