@@ -146,9 +146,13 @@ __device__ __forceinline__ int up_groups(int pxy, int pz) {
 // points along the third side per thread.
 template <typename R, int SW>
 struct UpSmem {
-  R L[3][kP + 2][kUpTile];  // two spare rows: the last group of LC rows may run past kP
-  R D[3][kP + 2][kUpTile];  // derivative along the side times the normal component
-  R S[kUpTile][SW];
+  // per side and source: (L_q, D_q), D the derivative along the side times the
+  // normal component.  Grid points side by side, so that the threads of a warp
+  // (neighbouring grid points, one source) read without bank conflicts; the
+  // row length keeps the writes (one source per lane) free of them too and
+  // leaves room for the last group of LC points to run past kP.
+  typename Vec<R>::T2 B[3][kUpTile][kP + 3];
+  __align__(16) R S[kUpTile][SW];
 };
 
 template <int KIND, typename R, bool SIG, int LC>
@@ -159,8 +163,8 @@ __device__ __forceinline__ void tree_up_body(const UpItemD& it, const TreeArgs& 
                                              UpSmem<R, KIND == 1 ? 4 : 2>& sm) {
   constexpr int SW = KIND == 1 ? 4 : 2;
   constexpr int C = KIND == 1 ? 2 : 1;
-  auto& sL = sm.L;
-  auto& sD = sm.D;
+  using R2 = typename Vec<R>::T2;
+  auto& sB = sm.B;
   auto& sS = sm.S;
   const int m = blockIdx.y, tid = threadIdx.x;
   const int npd[3] = {it.np0, it.np1, it.np2};
@@ -200,8 +204,7 @@ __device__ __forceinline__ void tree_up_body(const UpItemD& it, const TreeArgs& 
 #pragma unroll
           for (int q = 0; q < kP; ++q)
             if (q < npd[d]) {
-              sL[d][q][s] = L[q];
-              sD[d][q][s] = D[q] * sc;
+              sB[d][s][q] = R2{L[q], D[q] * sc};
             }
         }
       }
@@ -227,13 +230,23 @@ __device__ __forceinline__ void tree_up_body(const UpItemD& it, const TreeArgs& 
       }
       __syncthreads();
       if (nl > 0) {
-        R tr[LC], ti[LC];
+        // FP32: tile sums in FP32, added to the FP64 sums after the tile
+        constexpr bool kTileSums = sizeof(R) == 4;
+        R trs[kTileSums ? LC : 1], tis[kTileSums ? LC : 1];
+        auto tr = [&](int l) -> R& {
+          if constexpr (kTileSums) return trs[l]; else return reinterpret_cast<R&>(accr[l]);
+        };
+        auto ti = [&](int l) -> R& {
+          if constexpr (kTileSums) return tis[l]; else return reinterpret_cast<R&>(acci[l]);
+        };
+        if constexpr (kTileSums) {
 #pragma unroll
-        for (int l = 0; l < LC; ++l) tr[l] = ti[l] = R(0);
+          for (int l = 0; l < LC; ++l) trs[l] = tis[l] = R(0);
+        }
 #pragma unroll 2
         for (int s = 0; s < ns; ++s) {
-          const R lx = sL[0][i][s], dx = sD[0][i][s], ly = sL[1][j][s], dy = sD[1][j][s];
-          const R v = lx * ly, gxy = fma(dx, ly, lx * dy);
+          const R2 bx = sB[0][s][i], by = sB[1][s][j];
+          const R v = bx.x * by.x, gxy = fma(bx.y, by.x, bx.x * by.y);
           R ar, ai = R(0), br, bi = R(0);
           if constexpr (KIND == 1) {
             ar = fma(sS[s][0], v, sS[s][2] * gxy);
@@ -247,15 +260,17 @@ __device__ __forceinline__ void tree_up_body(const UpItemD& it, const TreeArgs& 
           // a group's last l may lie beyond pz: its sums are not written
 #pragma unroll
           for (int l = 0; l < LC; ++l) {
-            const R lz = sL[2][l0 + l][s], dz = sD[2][l0 + l][s];
-            tr[l] = fma(ar, lz, fma(br, dz, tr[l]));
-            if constexpr (KIND == 1) ti[l] = fma(ai, lz, fma(bi, dz, ti[l]));
+            const R2 bz = sB[2][s][l0 + l];
+            tr(l) = fma(ar, bz.x, fma(br, bz.y, tr(l)));
+            if constexpr (KIND == 1) ti(l) = fma(ai, bz.x, fma(bi, bz.y, ti(l)));
           }
         }
+        if constexpr (kTileSums) {
 #pragma unroll
-        for (int l = 0; l < LC; ++l) {
-          accr[l] += double(tr[l]);
-          acci[l] += double(ti[l]);
+          for (int l = 0; l < LC; ++l) {
+            accr[l] += double(trs[l]);
+            acci[l] += double(tis[l]);
+          }
         }
       }
     }
