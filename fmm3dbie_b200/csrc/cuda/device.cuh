@@ -129,10 +129,14 @@ int far_nchunks(int64_t ntarg, int64_t nptso, int kind, int precision, int nd, i
 int far_variants();
 constexpr int kFarSmall = 5;  // one-density shape for few targets
 bool far_small_fits(int64_t ntarg, int nd);  // whether the autotuner tries it
-// Tensor-core far field (variants 3 and 4 of the multi-density FP32
-// Helmholtz path): densities per CTA, 0 where the variant does not apply.
+// Matrix-instruction far field (variants 3 and 4 of the multi-density
+// Helmholtz path; FP32 far_tc.cu, FP64 far_dmma.cu): densities per CTA, 0
+// where the variant does not apply.
 int far_tc_group(int variant, int nd, int precision, int kind);
-int far_tc_targets();  // targets per CTA
+int far_tc_targets(int precision);  // targets per CTA
+int far_dmma_targets();
+cudaError_t far_dmma(int group, const Geometry& g, const KParams& kp, const MatvecArgs& a,
+                     cudaStream_t st, int* occ);
 // Floats of a.tc_ops that every variant of (nd, precision, kind) fits in.
 size_t far_tc_operand_floats(int nd, int precision, int kind, int64_t nptso);
 // Launches it, or with occ != null reports its resident CTAs per SM.

@@ -624,16 +624,24 @@ cudaError_t far_tc_n(const Geometry& g, const KParams& kp, const MatvecArgs& a, 
 
 }  // namespace
 
-int far_tc_targets() { return kTcT; }
+int far_tc_targets(int precision) { return precision == 1 ? kTcT : far_dmma_targets(); }
 
 int far_tc_group(int variant, int nd, int precision, int kind) {
-  if (variant < 3 || variant > 4 || precision != 1 || kind != 1 || nd < 2) return 0;
+  if (variant < 3 || variant > 4 || kind != 1) return 0;
+  if (precision == 0) {
+    // FP64: from 9 densities, where the CUDA-core kernel holds fewer than a
+    // block here (at 4 and 8 the padding to 16 columns costs more)
+    if (variant == 4) return nd > 32 ? 32 : 0;
+    return nd <= 8 ? 0 : nd <= 16 ? 16 : nd <= 32 ? 32 : 64;
+  }
+  if (nd < 2) return 0;
   if (variant == 4) return nd > 32 ? 64 : 0;
   return nd <= 16 ? 16 : 32;
 }
 
 size_t far_tc_operand_floats(int nd, int precision, int kind, int64_t nptso) {
   size_t most = 0;
+  if (precision != 1) return 0;
   for (int v = 3; v <= 4; ++v) {
     const int n = far_tc_group(v, nd, precision, kind);
     if (n > 0) most = std::max(most, size_t((nd + n - 1) / n) * n);
@@ -643,7 +651,9 @@ size_t far_tc_operand_floats(int nd, int precision, int kind, int64_t nptso) {
 
 cudaError_t far_tc(int variant, const Geometry& g, const KParams& kp, const MatvecArgs& a,
                    cudaStream_t st, int* occ) {
-  switch (far_tc_group(variant, a.nd, a.precision, kp.kind)) {
+  const int group = far_tc_group(variant, a.nd, a.precision, kp.kind);
+  if (group > 0 && a.precision == 0) return far_dmma(group, g, kp, a, st, occ);
+  switch (group) {
     case 16:
       return far_tc_n<16>(g, kp, a, st, occ);
     case 32:

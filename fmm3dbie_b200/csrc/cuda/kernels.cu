@@ -2516,7 +2516,7 @@ int far_variants() { return kFarSmall + 1; }
 bool far_small_fits(int64_t ntarg, int nd) { return nd == 1 && ntarg <= kSmallMax; }
 
 int far_block_targets(int kind, int precision, int variant, int md, int nd) {
-  if (md && far_tc_group(variant, nd, precision, kind) > 0) return far_tc_targets();
+  if (md && far_tc_group(variant, nd, precision, kind) > 0) return far_tc_targets(precision);
   if (!md && variant == kFarSmall) return kSmallTargets;
   const int v = variant < 0 || variant > 2 ? 0 : variant;
   if (md) return kMdShapes[md_class(nd)][v][0] * md_tpt(kind, precision, md_class(nd), v);

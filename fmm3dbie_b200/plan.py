@@ -72,7 +72,8 @@ class Plan:
 
     def set_far(self, iprec: int, nd: int, variant: int, nchunks: int):
         """Pin the far-field shape of (iprec, nd) (variants 0-2 CUDA cores,
-        3-4 tensor cores for FP32 Helmholtz with nd >= 2)."""
+        3-4 matrix instructions for Helmholtz: FP32 with nd >= 2, FP64 with
+        nd > 8)."""
         L.check(L.lib().bie_plan_set_far(self._h, iprec, nd, variant, nchunks), "bie_plan_set_far")
 
     def get_far(self, iprec: int, nd: int):

@@ -379,9 +379,9 @@ int bie_get_oversample_engine(void);
 int bie_plan_oversample(void* plan, int64_t engine, int64_t nd, const double* sigma_dev,
                         float* out_dev, void* stream);
 /* Far-field shape of (iprec, nd): bie_plan_set_far pins it (variant 0-2:
- * CUDA-core block shapes; 3-4: tensor-core kernel of the FP32 Helmholtz
- * multi-density path, 16/32 or 64 densities per CTA, nd >= 2; nchunks source
- * chunks) instead of the autotuner's choice; bie_plan_get_far returns the
+ * CUDA-core block shapes; 3-4: matrix-instruction kernels of the Helmholtz
+ * multi-density path, 16/32 or 64 densities per CTA: tensor cores in FP32 for
+ * nd >= 2, FP64 matrix instructions for nd > 8; nchunks source chunks) instead of the autotuner's choice; bie_plan_get_far returns the
  * variant, the chunk count and a nonzero flag if a tensor-core launch timed
  * out waiting for its MMAs.  No reference counterpart. */
 int bie_plan_set_far(void* plan, int64_t iprec, int64_t nd, int64_t variant, int64_t nchunks);
