@@ -1345,6 +1345,119 @@ __global__ void __launch_bounds__(kCombineThreads, kCombineBlocks<MODE>)
   combine_rows<CPLX, W, MODE>(g, nr, weff, sigma, partial, nchunks, pot, nd, blockIdx.x);
 }
 
+// Near correction of more than 8 complex densities with FP64 matrix
+// instructions (mma.m8n8k4.f64): one warp takes 8 consecutive rows (targets of
+// one patch, mostly with the same near patches) and N densities and walks the
+// union of the rows' near patches; per step of 4 nodes lane (row, node) =
+// (lane / 4, lane % 4) holds its row's W_eff entry (zero where the row lacks the
+// patch) as its element of A, and the nodes' densities are the B operands, so a
+// density is read once for 8 rows instead of once a row and a W_eff entry is
+// converted once instead of by every lane.  Heads of the rows' lists are taken
+// in ascending patch order; lists in any order are covered, each entry once.
+// 36,504 rows: 0.98 -> 0.42 ms at 64 densities, 0.41 -> 0.16 at 16 (FP32
+// W_eff); blocks of 32 and 64 densities (0.57 and 0.52 ms at 64) leave fewer
+// warps to hide the loads.
+__device__ __forceinline__ void dmma884(double* c, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+
+constexpr int kCombineMmaThreads = 128, kCombineMmaN = 16;
+// Warps from which it is used: 469 warps (3,750 rows, 16 densities) measured
+// 0.072 against 0.053 ms of the wide form, which has one warp a row; 1,876
+// warps (64 densities) 0.084 against 0.114.
+constexpr int64_t kCombineMmaWarps = 1536;
+
+template <typename W>
+__global__ void __launch_bounds__(kCombineMmaThreads)
+    combine_mma_kernel(Geometry g, Near nr, const W* __restrict__ weff,
+                       const double2* __restrict__ sigma, const double2* __restrict__ partial,
+                       int nchunks, double2* __restrict__ pot, int nd) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int N = kCombineMmaN;
+  const int lane = threadIdx.x & 31, row = lane >> 2, src = lane & 3;
+  const int64_t group = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int64_t i = 8 * group + row;
+  if (8 * group >= g.ntarg) return;  // whole warps
+  const int m0 = int(blockIdx.y) * N;
+  const bool in = i < g.ntarg;
+  int64_t k = in ? nr.row_ptr[i] : 0;
+  const int64_t k1 = in ? nr.row_ptr[i + 1] : 0;
+  double re[N / 8][2], im[N / 8][2];
+  // far-field partial sums: this lane's row, densities 8 j + 2 src, + 1
+#pragma unroll
+  for (int j = 0; j < N / 8; ++j)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      double ar = 0.0, ai = 0.0;
+      const int m = m0 + 8 * j + 2 * src + c;
+      if (in && m < nd)
+        for (int q = 0; q < nchunks; ++q) {
+          const double2 v = partial[(size_t(q) * g.ntarg + i) * nd + m];
+          ar += v.x;
+          ai += v.y;
+        }
+      re[j][c] = ar;
+      im[j][c] = ai;
+    }
+  constexpr int kNone = 0x7fffffff;
+  int head = k < k1 ? nr.col[k] : kNone;
+  for (;;) {
+    const int p = __reduce_min_sync(kFull, head);
+    if (p == kNone) break;
+    const bool mine = head == p;
+    const int64_t wo = mine ? nr.wofs[k] : 0;
+    if (mine) head = ++k < k1 ? nr.col[k] : kNone;
+    const int ps = g.pstart[p], np = g.pstart[p + 1] - ps;
+#pragma unroll 2
+    for (int st = 0; st < np; st += 4) {
+      const int node = st + src;
+      double wr = 0.0, wi = 0.0;
+      if (mine && node < np) {
+        const typename Vec2<W>::T w = reinterpret_cast<const typename Vec2<W>::T*>(weff)[wo + node];
+        wr = double(w.x);
+        wi = double(w.y);
+      }
+      const double mi = -wi;
+      const double2* sp = sigma + size_t(ps + min(node, np - 1)) * nd + m0 + row;
+#pragma unroll
+      for (int j = 0; j < N / 8; ++j) {
+        double2 d = make_double2(0.0, 0.0);
+        if (m0 + 8 * j + row < nd) d = sp[8 * j];
+        dmma884(re[j], wr, d.x);
+        dmma884(im[j], wr, d.y);
+        dmma884(re[j], mi, d.y);
+        dmma884(im[j], wi, d.x);
+      }
+    }
+  }
+  if (!in) return;
+#pragma unroll
+  for (int j = 0; j < N / 8; ++j)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int m = m0 + 8 * j + 2 * src + c;
+      if (m < nd) pot[size_t(i) * nd + m] = make_double2(re[j][c], im[j][c]);
+    }
+}
+
+int64_t combine_mma_warps(int64_t ntarg, int nd) {
+  return ((ntarg + 7) / 8) * ((nd + kCombineMmaN - 1) / kCombineMmaN);
+}
+
+template <typename W>
+void launch_combine_mma(const Geometry& g, const Near& nr, const W* w, const MatvecArgs& a,
+                        cudaStream_t st) {
+  const int64_t warps = (g.ntarg + 7) / 8;
+  const unsigned blocks = unsigned((warps * 32 + kCombineMmaThreads - 1) / kCombineMmaThreads);
+  combine_mma_kernel<W>
+      <<<dim3(blocks, unsigned((a.nd + kCombineMmaN - 1) / kCombineMmaN)), kCombineMmaThreads, 0, st>>>(
+          g, nr, w, reinterpret_cast<const double2*>(a.sigma),
+          reinterpret_cast<const double2*>(a.partial), a.nchunks,
+          reinterpret_cast<double2*>(a.pot), a.nd);
+}
+
 // ---------------------------------------------------------------------------
 // fold: W_eff = wnear - (smooth oversampled contribution) for each near pair
 //
@@ -2578,6 +2691,15 @@ cudaError_t launch_combine(const Geometry& g, const Near& nr, const KParams& kp,
   };
   const float* wf = static_cast<const float*>(a.weff);
   const double* wd = static_cast<const double*>(a.weff);
+  if (kp.kind == 1 && combine_mode(a.nd) == kCombineWide &&
+      combine_mma_warps(g.ntarg, a.nd) >= kCombineMmaWarps) {
+    if (a.weff_f32)
+      launch_combine_mma(g, nr, wf, a, st);
+    else
+      launch_combine_mma(g, nr, wd, a, st);
+    count();
+    return cudaGetLastError();
+  }
   if (kp.kind == 1) {
     if (a.weff_f32)
       by_mode(combine_kernel<1, float, 0>, combine_kernel<1, float, 1>,
