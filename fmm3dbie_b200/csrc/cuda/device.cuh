@@ -213,6 +213,9 @@ struct GivensArgs {
   int64_t* done = nullptr;
   int* brk = nullptr;
   double *errs = nullptr, *scale = nullptr;
+  // host memory that the device can write (one system only, may be null): set
+  // to 2 (it + 1) + (1 if the system is done) by the step
+  int64_t* status = nullptr;
 };
 // One pass of the orthogonalisation: w -= sum_k hsub[k] Vsub_k for k < msub
 // (if hsub), then out = the inner products of launch_mdot with the m vectors
@@ -222,11 +225,20 @@ cudaError_t launch_orth(const double* V, int64_t ldv, int m, double* w, const do
                         int cplx, const Segs& sg, double* partial, double* out,
                         const double* hsub, int msub, const double* Vsub, const GivensArgs* gv,
                         cudaStream_t st);
+// Whether launch_orth_cluster takes a single system of n nodes against m
+// vectors, and that call: both Gram-Schmidt passes, the norm, the Givens step
+// (its h1, h2 and nrm are not used) and vnext = w / ||w|| in one launch; w
+// keeps its value.
+bool orth_cluster_fits(int64_t n, int m);
+cudaError_t launch_orth_cluster(const double* V, int64_t ldv, int m, const double* w,
+                                const double* wts, int64_t n, int cplx, double* vnext,
+                                const GivensArgs& gv, cudaStream_t st);
 // State at the start of a solve from the squared norms of the residual and
-// (with an initial guess) of the right-hand side.
+// (with an initial guess) of the right-hand side (status: 0, or 1
+// for a zero residual).
 cudaError_t launch_gmres_init(int M, int nsys, const double* nrm, const double* nrmb,
                               double* scale, double* sv, double* bnorm, int64_t* done, int* brk,
-                              cudaStream_t st);
+                              int64_t* status, cudaStream_t st);
 cudaError_t launch_gmres_backsolve(int M, int nsys, int mused, const double* H, const double* sv,
                                    const int64_t* done, double* coef, cudaStream_t st);
 // Krylov-basis coefficients (mcols per system) of each system's GMRES

@@ -11,6 +11,7 @@
 //   (c) combine   : pot_i = sum of far partials + sum_k W_eff(k) . sigma,
 //                   W_eff = wnear - smooth near part (folded once per plan,
 //                   replacing the per-call l3ddirectcdp/h3ddirectcdp subtraction).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1749,9 +1750,16 @@ __device__ __forceinline__ void givens_step(const GivensArgs& g, int q, int lane
   if (err <= g.eps[q] || it == M - 1 || wnrm == 0.0) g.done[q] = it + 1;
 }
 
+// The step and, if the host polls for it, its outcome.
+__device__ __forceinline__ void givens_report(const GivensArgs& g, int q, int lane) {
+  givens_step(g, q, lane);
+  if (lane == 0 && g.status)
+    *static_cast<volatile int64_t*>(g.status) = 2 * int64_t(g.it + 1) + (g.done[q] != 0 ? 1 : 0);
+}
+
 __global__ void gmres_givens_kernel(GivensArgs g) {
   const int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (q < g.nsys) givens_step(g, q, threadIdx.x & 31);
+  if (q < g.nsys) givens_report(g, q, threadIdx.x & 31);
 }
 
 // out[2 b] = sum over the segment's chunks of the partials of b = (k, sys),
@@ -1898,8 +1906,160 @@ __global__ void orth_kernel(const double* V, int64_t ldv, int m, double* w,
     if (gv.nsys > 0) {
       __syncthreads();
       if (warp < nw)
-        for (int q = warp; q < gv.nsys; q += nw) givens_step(gv, q, lane);
+        for (int q = warp; q < gv.nsys; q += nw) givens_report(gv, q, lane);
     }
+  }
+}
+
+// The whole orthogonalisation of one small system in one launch: both
+// Gram-Schmidt passes, the norm, the Givens step and the next basis vector
+// vnext = w / ||w||, by one cluster of kOrthCluster blocks that keeps w in
+// shared memory (a slice of the nodes each) and adds up the slices' inner
+// products through distributed shared memory, every block in the same order.
+// Latency bounds it: four cluster barriers, the rotation chain (3 us) and,
+// for larger systems, 8 SMs' share of the L2 bandwidth (V is read once from
+// L2 and three times from L1 where a block's slice fits).  An iteration of 24
+// on average, against three launches of orth_kernel and a scaling (without
+// the gaps between those): 600 complex nodes 25.8 -> 13.5 us, 5,760 29.7 ->
+// 17.9, 16,128 42.3 -> 30.3, 31,360 50.0 -> 48.2.  1, 2 and 4 blocks: 16.5,
+// 15.0, 13.8 us at 600 nodes, 56, 34, 24 at 5,760.
+constexpr int kOrthCluster = 8, kOrthThreads = 1024, kOrthCols = 64;
+
+template <int CPLX>
+__global__ void __launch_bounds__(kOrthThreads, 1)
+    orth_cluster_kernel(const double* V, int64_t ldv, int m, const double* __restrict__ w,
+                        const double* __restrict__ wts, int n, double* vnext, GivensArgs gv) {
+  namespace cg = cooperative_groups;
+  constexpr int kWarps = kOrthThreads / 32;
+  extern __shared__ double2 s_dyn[];
+  __shared__ double2 s_part[kWarps > kOrthCols ? kWarps : kOrthCols];  // of this block
+  __shared__ double2 s_slot[3][kOrthCluster][kOrthCols];               // of all blocks
+  __shared__ double2 s_h[2][kOrthCols];
+  __shared__ double s_nrm[2];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = int(cluster.block_rank());
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int per = (n + kOrthCluster - 1) / kOrthCluster;
+  const int lo = min(n, rank * per), len = min(n, lo + per) - lo;
+  double2* sx = s_dyn;  // the slice of w (real: .x only), then its node weights
+  double* swt = reinterpret_cast<double*>(s_dyn + per);
+  for (int e = tid; e < len; e += kOrthThreads) {
+    if (CPLX)
+      sx[e] = reinterpret_cast<const double2*>(w)[lo + e];
+    else
+      sx[e] = make_double2(w[lo + e], 0.0);
+    swt[e] = wts[lo + e];
+  }
+  cluster.sync();  // every block runs before its memory is written
+  // a warp takes (vector k, 1 of `parts` parts of the slice)
+  const int parts = m < kWarps ? kWarps / m : 1;
+  auto warp_sum = [&](double2 v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+      if (CPLX) v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+    }
+    return v;
+  };
+  auto gather = [&](int which, int cols) {  // s_part[cols] of every block into s_slot[which]
+    for (int i = tid; i < cols * kOrthCluster; i += kOrthThreads) {
+      const int k = i / kOrthCluster, b = i % kOrthCluster;
+      *cluster.map_shared_rank(&s_slot[which][rank][k], b) = s_part[k];
+    }
+    cluster.sync();
+  };
+  auto total = [&](int which, int k) {
+    double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int b = 0; b < kOrthCluster; ++b) {
+      t.x += s_slot[which][b][k].x;
+      t.y += s_slot[which][b][k].y;
+    }
+    return t;
+  };
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int i = warp; i < m * parts; i += kWarps) {
+      const int k = i / parts, part = i % parts;
+      const double* v = V + size_t(k) * ldv;
+      double2 acc = make_double2(0.0, 0.0);
+#pragma unroll 4
+      for (int e = part * 32 + lane; e < len; e += 32 * parts) {
+        const double2 x = sx[e];
+        const double wt = swt[e];
+        if (CPLX) {
+          const double2 b = reinterpret_cast<const double2*>(v)[lo + e];
+          acc.x += wt * (b.x * x.x + b.y * x.y);
+          acc.y += wt * (b.x * x.y - b.y * x.x);
+        } else {
+          acc.x += wt * v[lo + e] * x.x;
+        }
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) s_part[i] = acc;
+    }
+    __syncthreads();
+    if (parts > 1) {  // m <= 16 vectors
+      double2 t = make_double2(0.0, 0.0);
+      if (tid < m)
+        for (int p = 0; p < parts; ++p) {
+          t.x += s_part[tid * parts + p].x;
+          t.y += s_part[tid * parts + p].y;
+        }
+      __syncthreads();
+      if (tid < m) s_part[tid] = t;
+      __syncthreads();
+    }
+    gather(pass, m);
+    if (tid < m) s_h[pass][tid] = total(pass, tid);
+    __syncthreads();
+    for (int e = tid; e < len; e += kOrthThreads) {
+      double2 x = sx[e];
+#pragma unroll 4
+      for (int k = 0; k < m; ++k) {
+        const double2 h = s_h[pass][k];
+        if (CPLX) {
+          const double2 v = reinterpret_cast<const double2*>(V + size_t(k) * ldv)[lo + e];
+          x.x -= h.x * v.x - h.y * v.y;
+          x.y -= h.x * v.y + h.y * v.x;
+        } else {
+          x.x -= h.x * V[size_t(k) * ldv + lo + e];
+        }
+      }
+      sx[e] = x;
+    }
+    __syncthreads();
+  }
+  {
+    double2 acc = make_double2(0.0, 0.0);
+    for (int e = tid; e < len; e += kOrthThreads)
+      acc.x += swt[e] * (sx[e].x * sx[e].x + sx[e].y * sx[e].y);
+    acc = warp_sum(acc);
+    if (lane == 0) s_part[warp] = acc;
+    __syncthreads();
+    if (warp == 0) {
+      acc = warp_sum(lane < kWarps ? s_part[lane] : make_double2(0.0, 0.0));
+      if (lane == 0) s_part[0] = acc;
+    }
+    __syncthreads();
+    gather(2, 1);  // the last access to another block's memory
+  }
+  const double nrm = total(2, 0).x;
+  const double root = sqrt(fmax(nrm, 0.0));
+  const double sc = root > 0.0 ? 1.0 / root : 0.0;
+  if (rank == 0 && warp == 0) {
+    if (lane == 0) s_nrm[0] = nrm;
+    __syncwarp();
+    GivensArgs g = gv;
+    g.h1 = reinterpret_cast<const double*>(s_h[0]);
+    g.h2 = reinterpret_cast<const double*>(s_h[1]);
+    g.nrm = s_nrm;
+    givens_report(g, 0, lane);
+  }
+  for (int e = tid; e < len; e += kOrthThreads) {
+    if (CPLX)
+      reinterpret_cast<double2*>(vnext)[lo + e] = make_double2(sc * sx[e].x, sc * sx[e].y);
+    else
+      vnext[lo + e] = sc * sx[e].x;
   }
 }
 
@@ -2825,6 +2985,47 @@ cudaError_t launch_orth(const double* V, int64_t ldv, int m, double* w, const do
   return cudaGetLastError();
 }
 
+// One system takes the cluster form up to this many nodes and values of the
+// basis: the chip-wide form costs about 33 us (three gaps included) + 0.064 ns
+// a value, this one 11 us + 0.094 ns.
+constexpr int64_t kOrthClusterNodes = 16384, kOrthClusterValues = int64_t(1) << 19;
+
+bool orth_cluster_fits(int64_t n, int m) {
+  return n <= kOrthClusterNodes && m <= kOrthCols && n * m <= kOrthClusterValues;
+}
+
+cudaError_t launch_orth_cluster(const double* V, int64_t ldv, int m, const double* w,
+                                const double* wts, int64_t n, int cplx, double* vnext,
+                                const GivensArgs& gv, cudaStream_t st) {
+  auto go = [&](auto kern) {
+    const int64_t per = (n + kOrthCluster - 1) / kOrthCluster;
+    const size_t smem = size_t(per) * (sizeof(double2) + sizeof(double));
+    if (smem > 16 * 1024) {  // beyond 48 KB with the static arrays
+      const cudaError_t e = cudaFuncSetAttribute(
+          kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+          int(kOrthClusterNodes / kOrthCluster * (sizeof(double2) + sizeof(double))));
+      if (e != cudaSuccess) return e;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kOrthCluster);
+    cfg.blockDim = dim3(kOrthThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kOrthCluster;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, V, ldv, m, w, wts, int(n), vnext, gv);
+  };
+  const cudaError_t e = cplx ? go(orth_cluster_kernel<1>) : go(orth_cluster_kernel<0>);
+  if (e != cudaSuccess) return e;
+  count();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_mdot(const double* V, int64_t ldv, int m, const double* w, const double* wts,
                         int nd, int cplx, const Segs& sg, double* partial, double* out,
                         cudaStream_t st) {
@@ -2870,7 +3071,8 @@ cudaError_t launch_axpbys(const double* x, double* y, const double* a, double br
 __global__ void gmres_init_kernel(int M, int nsys, const double* __restrict__ nrm,
                                   const double* __restrict__ nrmb, double* __restrict__ scale,
                                   double* __restrict__ sv, double* __restrict__ bnorm,
-                                  int64_t* __restrict__ done, int* __restrict__ brk) {
+                                  int64_t* __restrict__ done, int* __restrict__ brk,
+                                  int64_t* status) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nsys) return;
   // (a NaN stays one: the first Givens step reports it)
@@ -2881,13 +3083,14 @@ __global__ void gmres_init_kernel(int M, int nsys, const double* __restrict__ nr
   bnorm[q] = nrmb ? root(nrmb[2 * q]) : rb;
   done[q] = rb == 0.0 ? -1 : 0;
   brk[q] = 0;
+  if (status) *static_cast<volatile int64_t*>(status) = done[q] != 0 ? 1 : 0;
 }
 
 cudaError_t launch_gmres_init(int M, int nsys, const double* nrm, const double* nrmb,
                               double* scale, double* sv, double* bnorm, int64_t* done, int* brk,
-                              cudaStream_t st) {
+                              int64_t* status, cudaStream_t st) {
   gmres_init_kernel<<<(nsys + 63) / 64, 64, 0, st>>>(M, nsys, nrm, nrmb, scale, sv, bnorm, done,
-                                                     brk);
+                                                     brk, status);
   count();
   return cudaGetLastError();
 }

@@ -138,6 +138,21 @@ struct PlanSpec {
   bool async_weff = false;
 };
 
+// One word of pinned host memory that kernels write and the host polls.
+struct HostWord {
+  int64_t* p = nullptr;
+  HostWord() = default;
+  HostWord(const HostWord&) = delete;
+  HostWord& operator=(const HostWord&) = delete;
+  ~HostWord() {
+    if (p) cudaFreeHost(p);
+  }
+  cudaError_t alloc() {
+    return p ? cudaSuccess
+             : cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int64_t), cudaHostAllocPortable);
+  }
+};
+
 struct GmresWorkspace {
   DBuf<double> V, w, partial, dots, coef, scale;
   // least squares on the device: Hessenberg columns, rotations, residual
@@ -146,6 +161,7 @@ struct GmresWorkspace {
   DBuf<int64_t> done;
   DBuf<int> brk;
   DBuf<double> zc;  // Krylov-basis coefficients of the residual vector
+  HostWord status;  // of a single system's last Givens step
 };
 
 struct MixedWorkspace {

@@ -34,6 +34,22 @@ std::vector<double> interleave(const std::vector<cdouble>& v) {
   return o;
 }
 
+// Waits until a kernel in stream st has written *word >= least; a stream that
+// ends without it (an error) ends the wait.  The stop flag of an iteration by
+// a copy and a stream synchronisation took 26 us from the Givens step to the
+// next matvec's first kernel, this 8.
+cudaError_t poll_word(const volatile int64_t* word, int64_t least, cudaStream_t st) {
+  for (int spin = 1; *word < least; ++spin) {
+    if (spin % 4096) continue;
+    const cudaError_t e = cudaStreamQuery(st);
+    if (e == cudaErrorNotReady) continue;
+    if (e != cudaSuccess) return e;
+    return *word < least ? cudaErrorUnknown : cudaSuccess;
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return cudaSuccess;
+}
+
 }  // namespace
 
 int Operator::init_segments(cudaStream_t st) {
@@ -143,6 +159,13 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
   BIE_CUDA(ws.ls.alloc(nH + 2 * nR + nS + size_t(nsys) + nE));
   BIE_CUDA(ws.done.alloc(nsys));
   BIE_CUDA(ws.brk.alloc(nsys));
+  // a single system's stop flag is polled, those of several are copied
+  int64_t* status = nullptr;
+  if (nsys == 1) {
+    BIE_CUDA(ws.status.alloc());
+    status = ws.status.p;
+    *status = -1;
+  }
   double* d_H = ws.ls.p;
   double* d_cs = d_H + nH;
   double* d_sn = d_cs + nR;
@@ -151,11 +174,21 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
   double* d_errs = d_bnorm + nsys;
   BIE_CUDA(cudaMemsetAsync(d_errs, 0, nE * sizeof(double), st));
   BIE_CUDA(dev::launch_gmres_init(int(M), nsys, d_nrm, d_x0 ? d_h1 : nullptr, ws.scale.p, d_sv,
-                                  d_bnorm, ws.done.p, ws.brk.p, st));
+                                  d_bnorm, ws.done.p, ws.brk.p, status, st));
   BIE_CUDA(dev::launch_dscale(V, V, ws.scale.p, n, nd, cplx, sg, st));
   std::vector<int64_t> done(nsys, 0);
-  BIE_CUDA(cudaMemcpyAsync(done.data(), ws.done.p, nsys * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-  BIE_CUDA(cudaStreamSynchronize(st));
+  // stop flags after `step` iterations (0: the start)
+  auto read_done = [&](int64_t step) -> int {
+    if (status) {
+      BIE_CUDA(poll_word(status, 2 * step, st));
+      if (*static_cast<volatile int64_t*>(status) & 1) done[0] = step > 0 ? step : -1;
+      return kOk;
+    }
+    BIE_CUDA(cudaMemcpyAsync(done.data(), ws.done.p, nsys * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    BIE_CUDA(cudaStreamSynchronize(st));
+    return kOk;
+  };
+  if (int ier = read_done(0)) return ier;
   int nactive = 0;
   for (int q = 0; q < nsys; ++q) nactive += done[q] == 0 ? 1 : 0;
   out.niter.assign(nsys, 0);
@@ -195,14 +228,18 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
     gv.brk = ws.brk.p;
     gv.errs = d_errs;
     gv.scale = ws.scale.p;
+    gv.status = status;
     double* w = ws.w.p;
     double* pt = ws.partial.p;
-    BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h1, nullptr, 0, nullptr, nullptr, st));
-    BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h2, d_h1, m, V, nullptr, st));
-    BIE_CUDA(dev::launch_orth(w, ldv, 1, w, wts, nd, cplx, sg, pt, d_nrm, d_h2, m, V, &gv, st));
-    BIE_CUDA(dev::launch_dscale(ws.w.p, vnext, ws.scale.p, n, nd, cplx, sg, st));
-    BIE_CUDA(cudaMemcpyAsync(done.data(), ws.done.p, nsys * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    BIE_CUDA(cudaStreamSynchronize(st));
+    if (nsys == 1 && dev::orth_cluster_fits(n, m)) {
+      BIE_CUDA(dev::launch_orth_cluster(V, ldv, m, w, wts, n, cplx, vnext, gv, st));
+    } else {
+      BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h1, nullptr, 0, nullptr, nullptr, st));
+      BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h2, d_h1, m, V, nullptr, st));
+      BIE_CUDA(dev::launch_orth(w, ldv, 1, w, wts, nd, cplx, sg, pt, d_nrm, d_h2, m, V, &gv, st));
+      BIE_CUDA(dev::launch_dscale(ws.w.p, vnext, ws.scale.p, n, nd, cplx, sg, st));
+    }
+    if ((ier = read_done(it + 1))) return ier;
     nactive = 0;
     for (int q = 0; q < nsys; ++q) nactive += done[q] == 0 ? 1 : 0;
   }
