@@ -994,7 +994,8 @@ constexpr int kCombineMinBlocks = 5;
 // range, two entries per lane in flight.  nd = 4: 0.20 ms on the 35,840-node
 // matvec against 0.63 ms with the lanes over densities (the wide form); at
 // nd = 16 the same scheme with one density per lane measured 0.72 against
-// 0.62 ms, so the wide form serves more than 8 densities.
+// 0.62 ms, so more than 8 densities go to the wide form or, in large plans,
+// to combine_mma_kernel.
 template <int CPLX, typename W, int kD>
 __device__ __forceinline__ void combine_row_md(const Geometry& g, const Near& nr,
                                                const W* __restrict__ weff,
