@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kEvBlock<PROXYT>, (kEvMinBlocks<KIND, R, PROXY
   using R4 = typename Vec<R>::T4;
   constexpr int SW = KIND == 1 ? 4 : 2;
   constexpr int C = KIND == 1 ? 2 : 1;
-  constexpr int NT = kEvBlock<PROXYT>, TILE = NT, NW = NT / 32;
+  constexpr int NT = kEvBlock<PROXYT>, TILE = NT;
   constexpr bool F32 = sizeof(R) == 4;
   __shared__ __align__(16) TileSmem<KIND, R, TILE> tile[2];
   __shared__ double2 stab[!F32 && KIND == 1 ? kFarTrigN : 1];
@@ -432,11 +432,9 @@ __global__ void __launch_bounds__(kEvBlock<PROXYT>, (kEvMinBlocks<KIND, R, PROXY
                cz = F32 ? 0.5 * (tn.lo[2] + tn.hi[2]) : 0.0;
   // this thread's target and its part of every tile
   const int nt = PROXYT ? min(NT, tn.np0 * tn.np1 * tn.np2 - int(k0)) : int(tn.e - tn.b);
-  const int tw = (nt + 31) / 32;            // warps of targets
-  const int parts = PROXYT ? 1 : NW / tw;   // parts of the tile
-  const int part = (tid >> 5) / tw;         // (parts or more: this warp only loads)
-  const int ti = tid - part * tw * 32;      // target of this thread
-  const bool act = ti < nt, work = part < parts;
+  const tree::EvalSlot slot = tree::eval_slot(nt, NT, !PROXYT, tid);
+  const int parts = slot.parts, part = slot.part, ti = slot.target;
+  const bool act = ti < nt, work = slot.work;
   double x = cx, y = cy, z = cz;
   if (act) {
     const int64_t q = PROXYT ? tn.tpoff + k0 + ti : tn.b + ti;
@@ -500,8 +498,10 @@ __global__ void __launch_bounds__(kEvBlock<PROXYT>, (kEvMinBlocks<KIND, R, PROXY
       acci += double(pi);
     }
   }
+  // One thread stores a target's sum: the spare warps of an item with fewer
+  // targets than threads carry repeated target indices and zero sums.
   if constexpr (PROXYT) {
-    if (!act) return;
+    if (!slot.writes) return;
     R* o = phi + (size_t(tn.tpoff + k0 + ti) * nd + m) * C;
     o[0] = R(accr);
     if constexpr (C == 2) o[1] = R(acci);
@@ -515,12 +515,12 @@ __global__ void __launch_bounds__(kEvBlock<PROXYT>, (kEvMinBlocks<KIND, R, PROXY
       __syncthreads();
       for (int p = 1; p < parts; ++p)
         if (part == 0) {
-          const double2 v = sred[tid + p * tw * 32];
+          const double2 v = sred[tid + p * slot.stride];
           accr += v.x;
           acci += v.y;
         }
     }
-    if (!act || part != 0) return;
+    if (!slot.writes) return;
     const int64_t o = (size_t(ta.tperm[tn.b + ti]) * nd + m) * C;
     partial[o] = accr;
     if constexpr (C == 2) partial[o + 1] = acci;

@@ -90,6 +90,33 @@ void traverse(const Tree& T, const Tree& S, const Params& prm, double sep_min,
 // 0 when every (target leaf, source leaf) pair is covered exactly once.
 int check_coverage(const Tree& T, const Tree& S, const std::vector<Interaction>& ia);
 
+// What thread tid of an evaluation block of nthreads threads does for an item
+// of nt targets (1 <= nt <= nthreads): the targets take whole warps, and where
+// `split` is set every further group of as many warps takes another part of
+// each source tile for the same targets.  Warps that make up no whole group
+// (or, without `split`, all but the first group) only load tiles; their target
+// index repeats one of a working warp, so only `writes` decides who stores a
+// target's sum: exactly one thread per target.
+struct EvalSlot {
+  int target = 0;       // target of the item, < nt only for the lanes that have one
+  int part = 0;         // part of every tile
+  int parts = 1;        // parts of a tile in this block
+  int stride = 0;       // threads between one part's thread and the next part's
+  bool work = false;    // evaluates its part
+  bool writes = false;  // stores the target's sum
+};
+constexpr EvalSlot eval_slot(int nt, int nthreads, bool split, int tid) {
+  EvalSlot s;
+  const int tw = (nt + 31) / 32;
+  s.stride = tw * 32;
+  s.parts = split ? nthreads / 32 / tw : 1;
+  s.part = (tid >> 5) / tw;
+  s.target = tid - s.part * s.stride;
+  s.work = s.part < s.parts;
+  s.writes = s.part == 0 && s.target < nt;
+  return s;
+}
+
 // Chebyshev points of the second kind on [-1, 1], cos(pi j / (p - 1))
 // (the single point 0 when p = 1), and the Lagrange normalisations
 // 1 / prod_{i != j} (x_j - x_i).
