@@ -30,7 +30,8 @@
 //               of the CUDA-core kernels, so that the error-matched W_eff32
 //               fold still cancels their near-pair values; and the sums: each
 //               thread adds N / 2 columns of its target into FP32 registers
-//               after every tile and every kTcFold tiles into FP64 ones;
+//               after every tile and every kTcFold tiles into FP64 ones (64
+//               densities: into FP32 sums in shared memory, compensated);
 //   warp 16     producer: bulk copy of B, the tile's source coordinates;
 //   warp 17     issues the MMAs (the warp runs uniformly, one elected lane
 //               issues: from a single-lane branch the operands had to be
@@ -68,7 +69,6 @@ constexpr int kTcS = 64;           // sources per tile
 constexpr int kTcWarps = 16;       // warps that evaluate kernel values
 constexpr int kTcThreads = 32 * (kTcWarps + 2);
 constexpr int kTcPer = kTcS * 4 / kTcWarps;  // sources of a tile per thread
-constexpr int kTcStages = 3;       // source tiles in flight
 constexpr int kTcFold = 8;         // tiles summed in the first set of registers
 constexpr int kTcACols = 4 * kTcS; // tensor-memory columns of A: Kr hi, Ki hi, Kr lo, Ki lo
 constexpr uint32_t kTcTmemCols = 512;
@@ -96,11 +96,17 @@ struct TcGeom {
   int check, pad[3];
 };
 
+// Source tiles in flight; at 64 densities two, whose place the running sums
+// take (a tile's MMAs take five times as long as its copy).
+template <int N>
+constexpr int kTcStages = N == 64 ? 2 : 3;
+
 template <int N>
 struct TcSmem {
-  float b[kTcStages][kTcOpFloats<N>];
-  TcGeom geom[kTcStages];
-  uint64_t full[kTcStages], empty[kTcStages], afull, done;
+  float b[kTcStages<N>][kTcOpFloats<N>];
+  TcGeom geom[kTcStages<N>];
+  float run[N == 64 ? 2 * N * 4 / kTcWarps : 1][N == 64 ? 32 * kTcWarps : 1];  // running sums
+  uint64_t full[kTcStages<N>], empty[kTcStages<N>], afull, done;
   uint32_t tmem;
   int fail;
 };
@@ -273,6 +279,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   constexpr int SPLIT = kTcSplit<N>;
   static_assert(SPLIT * 2 * NB + kTcACols <= int(kTcTmemCols), "tensor memory");
   constexpr bool kTwoSums = N < 64;       // a second set of sums (64 densities: no registers left)
+  constexpr int ST = kTcStages<N>;
   constexpr uint32_t kLboB = (NB / 8) * 128;
   constexpr uint32_t kOpBytes = kTcOpFloats<N> * sizeof(float);
   extern __shared__ __align__(1024) unsigned char tc_smem[];
@@ -300,7 +307,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     auto init = [](uint64_t* b, int n) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n));
     };
-    for (int s = 0; s < kTcStages; ++s) {
+    for (int s = 0; s < ST; ++s) {
       init(&sm.full[s], 1);
       init(&sm.empty[s], kTcWarps + 1);
     }
@@ -345,10 +352,26 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
       }
     };
+    // 64 densities: the sums so far into the running sums in shared memory; what
+    // the addition rounds off (Knuth's TwoSum) starts the next sums, so that the
+    // error does not grow with the number of tiles
+    auto fold = [&]() {
+#pragma unroll
+      for (int n = 0; n < NH; ++n) {
+        float& v = n & 1 ? sum[n / 2].y : sum[n / 2].x;
+        float& r = sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid];
+        const float a = r, t = __fadd_rn(a, v), b = __fsub_rn(t, a);
+        v = __fadd_rn(__fsub_rn(a, __fsub_rn(t, b)), __fsub_rn(v, b));
+        r = t;
+      }
+    };
+    if (!kTwoSums)
+#pragma unroll
+      for (int n = 0; n < NH; ++n) sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid] = 0.f;
     const uint32_t a0 = acol + lanes + uint32_t(kTcPer * sgrp);
     for (int i = 0; i < ntiles; ++i) {
-      const int s = i % kTcStages;
-      ok = tc_wait_warp(&sm.full[s], uint32_t(i / kTcStages) & 1u, fail);
+      const int s = i % ST;
+      ok = tc_wait_warp(&sm.full[s], uint32_t(i / ST) & 1u, fail);
       if (!ok) break;
       const TcGeom& ge = sm.geom[s];
       float vr[kTcPer], vi[kTcPer];
@@ -391,6 +414,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) tc_arrive(&sm.afull);
+      if (!kTwoSums && i > 0 && i % kTcFold == 0) fold();  // under this tile's MMAs
     }
     if (ok && ntiles > 0) drain(ntiles - 1);
     if (ok && to < ntarg) {
@@ -401,7 +425,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (d0 + n < nd) {
           const double v = double(n & 1 ? sum[n / 2].y : sum[n / 2].x);
           partial[((size_t(blockIdx.y) * ntarg + to) * nd + d0 + n) * 2 + comp] =
-              kTwoSums ? sum2[kTwoSums ? n : 0] + v : v;
+              v + (kTwoSums ? sum2[kTwoSums ? n : 0]
+                            : double(sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid]));
         }
     }
   } else if (warp == kTcWarps) {
@@ -432,7 +457,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     if (ntiles > 0) fetch(s0);
     int issued = 0;
     for (int i = 0; i < ntiles; ++i) {
-      const int s = i % kTcStages;
+      const int s = i % ST;
       const int64_t sg = s0 + int64_t(i) * kTcS;
       float cur[H][6];
 #pragma unroll
@@ -448,7 +473,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const double g2 = gap * gap;
       const double gap2 = g2 + __shfl_down_sync(0xffffffffu, g2, 1) + __shfl_down_sync(0xffffffffu, g2, 2);
       if (i + 1 < ntiles) fetch(sg + kTcS);
-      if (i >= kTcStages && !tc_wait_warp(&sm.empty[s], uint32_t(i / kTcStages - 1) & 1u, fail)) break;
+      if (i >= ST && !tc_wait_warp(&sm.empty[s], uint32_t(i / ST - 1) & 1u, fail)) break;
       TcGeom& ge = sm.geom[s];
 #pragma unroll
       for (int h = 0; h < H; ++h) {
@@ -477,14 +502,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       issued = i + 1;
     }
     if (*fail)  // the copies still in flight land before the CTA goes
-      for (int i = issued > kTcStages ? issued - kTcStages : 0; i < issued; ++i)
+      for (int i = issued > ST ? issued - ST : 0; i < issued; ++i)
         for (uint32_t r = 0; r < kTcSpin; ++r) {
           uint32_t done;
           asm volatile(
               "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
               "selp.b32 %0, 1, 0, p;\n\t}\n"
               : "=r"(done)
-              : "r"(smem_u32(&sm.full[i % kTcStages])), "r"(uint32_t(i / kTcStages) & 1u)
+              : "r"(smem_u32(&sm.full[i % ST])), "r"(uint32_t(i / ST) & 1u)
               : "memory");
           if (done) break;
         }
@@ -495,8 +520,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint64_t bdesc = smem_desc(smem_u32(sm.b[0]), kLboB);
     int issued = -1;
     for (int i = 0; i < ntiles; ++i) {
-      const int s = i % kTcStages;
-      if (!tc_wait_warp(&sm.full[s], uint32_t(i / kTcStages) & 1u, fail)) break;
+      const int s = i % ST;
+      if (!tc_wait_warp(&sm.full[s], uint32_t(i / ST) & 1u, fail)) break;
       if (!tc_wait_warp(&sm.afull, uint32_t(i) & 1u, fail)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t bd = bdesc + uint64_t(uint32_t(s) * (kOpBytes >> 4));
