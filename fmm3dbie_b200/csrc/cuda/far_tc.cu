@@ -81,6 +81,21 @@ constexpr uint32_t kTcTmemCols = 512;
 template <int N>
 constexpr int kTcSplit = N == 64 ? 1 : (N == 32 ? 2 : 4);
 
+// What an accumulator loses: it cuts to 24 bits after each K = 8 step, so a sum
+// of n hi*hi steps comes out too small by about (n + 1) / 2 times the mean cut
+// of one rounding toward zero (0.72 units of 2^-24 for mantissas spread as those
+// of products are), more where the products themselves are cut to a large
+// accumulator's last place.  Measured against the CUDA-core kernel, in units of
+// 2^-24, on spheres, ellipsoids and tori of 864 to 36,504 nodes, k = 0.5 to 9 and
+// complex, single and double layers and both, random densities (the low ends)
+// and plane waves (the high ends): 2 steps 0.76 to 1.02, 4 steps 1.24 to 1.92,
+// 8 steps 2.2 to 4.5.  The sums are scaled up by the middle of the range, so
+// that what is left is below the CUDA-core kernel's own error (FP32 rsqrt, sine
+// and cosine: -3 to +1 units); without it, plane waves of k = 0.5 on a
+// 3,750-node sphere came out 1.4 times as far from FP64 as from that kernel.
+template <int N>
+constexpr double kTcLoss = (N == 64 ? 3.3 : N == 32 ? 1.6 : 0.9) / 16777216.0;
+
 constexpr uint32_t kTcSpin = 1u << 22;  // polls of one wait before the CTA gives up
 constexpr double kTcOver4Pi = 0.07957747154594767;
 static_assert(kFarTileSources % kTcS == 0, "chunks are whole tiles");
@@ -425,8 +440,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (d0 + n < nd) {
           const double v = double(n & 1 ? sum[n / 2].y : sum[n / 2].x);
           partial[((size_t(blockIdx.y) * ntarg + to) * nd + d0 + n) * 2 + comp] =
-              v + (kTwoSums ? sum2[kTwoSums ? n : 0]
-                            : double(sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid]));
+              (1.0 + kTcLoss<N>) *
+              (v + (kTwoSums ? sum2[kTwoSums ? n : 0]
+                             : double(sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid])));
         }
     }
   } else if (warp == kTcWarps) {
