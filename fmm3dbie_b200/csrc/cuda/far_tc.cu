@@ -210,7 +210,8 @@ __device__ __forceinline__ void tmem_store16(uint32_t addr, const float* v) {
 }
 
 // x -> high part (rounded to TF32) and remainder, which the tensor core reads
-// as TF32 (of its 12 significant bits at most the last one goes).
+// as TF32 (of its 12 significant bits at most the last one goes, the size of a
+// rounding of it; NaN for a NaN x).
 __device__ __forceinline__ void split_store16(uint32_t hi_addr, uint32_t lo_addr, float* v) {
   float hi[16];
 #pragma unroll

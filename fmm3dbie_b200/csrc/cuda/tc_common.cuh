@@ -20,7 +20,8 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 }
 
 // x rounded to TF32 (10 mantissa bits, ties away from zero) by integer
-// operations: add half of the dropped range, clear the low 13 bits.
+// operations: add half of the dropped range, clear the low 13 bits.  The
+// device's NaN (0x7fffffff) becomes -0: a caller keeps it in the low part.
 __device__ __forceinline__ float tf32_rn(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u);
 }
@@ -48,14 +49,20 @@ __device__ __forceinline__ int op_off(int r, int k, uint32_t lbo) {
   return (k >> 2) * int(lbo >> 2) + (r >> 3) * 32 + (r & 7) * 4;
 }
 
-// Four consecutive columns of one row, split into high and low parts
-// (hi = x rounded to TF32, lo = x - hi, exact, then rounded to TF32).
+// Low part of x beside hi = tf32_rn(x): x - hi, exact, rounded to TF32; NaN for
+// a NaN or infinite x, so that such a density reaches every product.
+__device__ __forceinline__ float tf32_lo(float x, float hi) {
+  const float d = x - hi;
+  return d == d ? tf32_rn(d) : d;
+}
+
+// Four consecutive columns of one row, split into high and low parts.
 __device__ __forceinline__ void store_split(float* hi, float* lo, int off, float a, float b,
                                             float c, float d) {
   const float ha = tf32_rn(a), hb = tf32_rn(b), hc = tf32_rn(c), hd = tf32_rn(d);
   *reinterpret_cast<float4*>(hi + off) = make_float4(ha, hb, hc, hd);
   *reinterpret_cast<float4*>(lo + off) =
-      make_float4(tf32_rn(a - ha), tf32_rn(b - hb), tf32_rn(c - hc), tf32_rn(d - hd));
+      make_float4(tf32_lo(a, ha), tf32_lo(b, hb), tf32_lo(c, hc), tf32_lo(d, hd));
 }
 
 // Bounded wait for phase `parity` of the barrier (thread 0 polls, the others
