@@ -79,7 +79,7 @@ __device__ __forceinline__ void pair_helm(double tx, double ty, double tz, const
   const double kr = k * r;
   double sn, cs;
   if (tab)
-    sincos_far(r, k * kFarTrigInvStep, tab, sn, cs);
+    sincos_far(kr, tab, sn, cs);
   else
     sincos(kr, &sn, &cs);
   double rs = rinv;
@@ -225,7 +225,7 @@ __device__ __forceinline__ void pair_helm_unit(double tx, double ty, double tz, 
   const double kr = k * r;
   double sn, cs;
   if (tab)
-    sincos_far(r, k * kFarTrigInvStep, tab, sn, cs);
+    sincos_far(kr, tab, sn, cs);
   else
     sincos(kr, &sn, &cs);
   double rs = rinv;
@@ -288,7 +288,7 @@ __device__ __forceinline__ void pair_charge(double tx, double ty, double tz, con
     const double r = r2 * rinv;
     double sn, cs;
     if (tab)
-      sincos_far(r, k * kFarTrigInvStep, tab, sn, cs);
+      sincos_far(k * r, tab, sn, cs);
     else
       sincos(k * r, &sn, &cs);
     double rs = rinv;

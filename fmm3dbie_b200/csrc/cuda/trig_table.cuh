@@ -42,30 +42,25 @@ __device__ __forceinline__ void sincos_tab(double x, const double2* tab, double&
 }
 
 // The far-field variant of the same method, for the direct and hierarchical
-// far-field kernels, whose phases stay below 100 and whose products only need
-// ~1e-14.  The FP64 pipe bounds those kernels, so the phase goes straight to
-// table steps and the table is fine enough for short series:
-//   u = k r N / (2 pi) = j + f, |f| <= 1/2, j by the round-to-integer of adding
-//   1.5 * 2^52 (no conversion instructions), f = u - j in one fused
-//   multiply-add (its error is the rounding of k N / (2 pi): 1.1e-16 of the
-//   phase);
-//   sin(2 pi f / N) to f^3, with the f^5 term economised on |f| <= 1/2
-//   (Lanczos: x^5 ~ 5/4 h^2 x^3 - 5/16 h^4 x on |x| <= h, error h^5 / 16), which
-//   leaves h^5 / 1920 = 1.4e-16 for h = pi / 1024; cos to f^4 (next term
-//   1.2e-18).
-// 12 FP64 operations; 256 entries with the series to rho^5 and rho^6 and a
-// separate phase k r took 15.
+// far-field kernels, whose phases k r stay below a few hundred (the surface in
+// wavelengths times 2 pi).  The FP64 pipe bounds those kernels, so the table is
+// fine enough for short series and nothing is converted:
+//   j = rint(x N / (2 pi)) by adding 1.5 * 2^52 (no conversion instructions),
+//   rho = x - j (2 pi / N) in one fused multiply-add with 2 pi / N rounded to
+//   FP64 (relative error 3.9e-17: the phase is off by as much of itself, a
+//   third of the rounding of k r),
+//   sin rho to rho^5 and cos rho to rho^4, |rho| <= pi / 1024: next terms
+//   rho^7 / 5040 = 5e-22 and rho^6 / 720 = 1.2e-18.
+// 13 FP64 operations; 256 entries took 15.  Distance of (sin, cos) from the true
+// values of k r: 2.0e-16 at most for phases up to 1 (256 entries: 2.4e-16), and
+// otherwise the rounding of k r, as there: 1.1e-14 up to 100.  (With the phase
+// taken straight to table steps, x = r (k N / (2 pi)), and a two-term sine it
+// was 12 operations, but 3.6e-16 up to 1, and the rounding of k N / (2 pi) moved
+// the whole wavenumber by up to 1.7e-16 of itself.)
 constexpr int kFarTrigN = 1024;
 constexpr double kFarTrigInvStep = 162.97466172610083;  // 1024 / (2 pi)
-constexpr double kRoundMagic = 6755399441055744.0;      // 1.5 * 2^52
 constexpr double kFarTrigStep = 0.006135923151542565;   // 2 pi / 1024
-constexpr double kFarTrigH = 0.5 * kFarTrigStep;
-constexpr double kFarS1 =
-    kFarTrigStep * (1.0 - 5.0 / 16.0 / 120.0 * kFarTrigH * kFarTrigH * kFarTrigH * kFarTrigH);
-constexpr double kFarS3 = kFarTrigStep * kFarTrigStep * kFarTrigStep *
-                          (-1.0 / 6.0 + 5.0 / 4.0 / 120.0 * kFarTrigH * kFarTrigH);
-constexpr double kFarC2 = -0.5 * kFarTrigStep * kFarTrigStep;
-constexpr double kFarC4 = kFarTrigStep * kFarTrigStep * kFarTrigStep * kFarTrigStep / 24.0;
+constexpr double kRoundMagic = 6755399441055744.0;      // 1.5 * 2^52
 
 // Fills tab[q] = (cos, sin)(2 pi q / N): the first octant by sincos (one
 // value a thread for 128 threads), the others by symmetry.  Ends with a
@@ -91,15 +86,13 @@ __device__ __forceinline__ void fill_far_trig_table(double2* tab) {
   __syncthreads();
 }
 
-// sin and cos of k r, kstep = k N / (2 pi).
-__device__ __forceinline__ void sincos_far(double r, double kstep, const double2* tab, double& s,
-                                           double& c) {
-  const double u = fma(r, kstep, kRoundMagic);
+__device__ __forceinline__ void sincos_far(double x, const double2* tab, double& s, double& c) {
+  const double u = fma(x, kFarTrigInvStep, kRoundMagic);
   const int j = __double2loint(u) & (kFarTrigN - 1);
-  const double f = fma(r, kstep, kRoundMagic - u);
-  const double f2 = f * f;
-  const double sp = f * fma(f2, kFarS3, kFarS1);
-  const double cp = fma(f2, fma(f2, kFarC4, kFarC2), 1.0);
+  const double rho = fma(kRoundMagic - u, kFarTrigStep, x);
+  const double r2 = rho * rho;
+  const double sp = fma(rho * r2, fma(r2, 1.0 / 120.0, -1.0 / 6.0), rho);
+  const double cp = fma(r2, fma(r2, 1.0 / 24.0, -0.5), 1.0);
   const double2 t = tab[j];
   s = fma(t.y, cp, t.x * sp);
   c = fma(t.x, cp, -(t.y * sp));
