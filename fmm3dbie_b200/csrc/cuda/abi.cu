@@ -1215,6 +1215,12 @@ int bie_plan_get_far(void* plan, int64_t iprec, int64_t nd, int64_t* out) {
   return BIE_OK;
 }
 
+int bie_plan_set_tc_wait(void* plan, int64_t polls) {
+  if (!plan || polls > int64_t(UINT32_MAX)) return BIE_ERR_ARG;
+  static_cast<bie::Plan*>(plan)->tc_spin = polls < 0 ? bie::dev::kTcSpin : uint32_t(polls);
+  return BIE_OK;
+}
+
 int bie_plan_set_far_method(void* plan, int64_t iprec, int64_t method, double theta, int64_t p,
                             int64_t leaf_t, int64_t leaf_s, void* stream) {
   if (!plan || (iprec != 0 && iprec != 1) || (method != 0 && method != 1)) return BIE_ERR_ARG;

@@ -75,6 +75,8 @@ struct KParams {
 
 // precision: 0 = f64 far field, 1 = f32 far field (f64 accumulation across
 // source tiles).
+constexpr uint32_t kTcSpin = 1u << 22;  // default of MatvecArgs::tc_spin
+
 struct MatvecArgs {
   int precision = 0;
   int nd = 1;
@@ -89,6 +91,7 @@ struct MatvecArgs {
   const void* ab = nullptr;       // per-source constants for the multi-density kernel
   float* tc_ops = nullptr;        // tensor-core far field: its density operand (far_tc_operand_floats)
   int* tc_err = nullptr;          // set by the tensor-core far field if a completion wait timed out
+  uint32_t tc_spin = kTcSpin;     // its limit of a wait, in polls
   const int32_t* sdest = nullptr; // strengths: source s is stored at position sdest[s]
 };
 

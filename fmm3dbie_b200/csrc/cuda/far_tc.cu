@@ -47,10 +47,13 @@
 // below that the kernel values with the operand splits (about 25 instructions
 // a pair; evaluation alone takes 3.4 of the 4.5 ms at 16 densities).
 //
-// Completion waits are bounded; on timeout the kernel records the CTA in
-// *err, every role leaves, the copies and MMAs in flight are waited for
-// (bounded), the tensor memory is freed and nothing is written.
+// Completion waits are bounded (MatvecArgs::tc_spin polls); on timeout the
+// kernel records the CTA in *err, every role leaves, the copies and MMAs in
+// flight are waited for (bounded), the tensor memory is freed and the CTA's sums
+// are NaN, so that no product goes on with what the buffer held before and a
+// solve ends with a breakdown.
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <cstdint>
@@ -96,7 +99,7 @@ constexpr int kTcSplit = N == 64 ? 1 : (N == 32 ? 2 : 4);
 template <int N>
 constexpr double kTcLoss = (N == 64 ? 3.3 : N == 32 ? 1.6 : 0.9) / 16777216.0;
 
-constexpr uint32_t kTcSpin = 1u << 22;  // polls of one wait before the CTA gives up
+constexpr uint32_t kTcDrain = 1u << 22;  // polls of a wait for work in flight at the end
 constexpr double kTcOver4Pi = 0.07957747154594767;
 static_assert(kFarTileSources % kTcS == 0, "chunks are whole tiles");
 
@@ -126,18 +129,23 @@ struct TcSmem {
   int fail;
 };
 
-// Waits (bounded) for phase `parity` of the barrier; false once any role of
-// the CTA has given up.
-__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* fail) {
-  for (uint32_t it = 0; it < kTcSpin; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
+__device__ __forceinline__ bool tc_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// Waits (at most `spin` polls) for phase `parity` of the barrier; false once any
+// role of the CTA has given up.
+__device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile int* fail,
+                                        uint32_t spin) {
+  for (uint32_t it = 0; it < spin; ++it) {
+    if (tc_try(bar, parity)) return true;
     if (*fail) return false;
   }
   *fail = 1;
@@ -145,8 +153,9 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
 }
 
 // The same for a whole warp, one answer for all lanes.
-__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail) {
-  return __all_sync(0xffffffffu, tc_wait(bar, parity, fail));
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* fail,
+                                             uint32_t spin) {
+  return __all_sync(0xffffffffu, tc_wait(bar, parity, fail, spin));
 }
 
 __device__ __forceinline__ void tc_arrive(uint64_t* bar) {
@@ -160,6 +169,7 @@ __device__ __forceinline__ void tc_arrive(uint64_t* bar) {
 struct TcConst {
   float2 k, kim, ar, ai, br, bi, mbr, one, mone;
   float thr2;
+  uint32_t spin;  // polls of a wait
 };
 
 template <bool CHECK, bool CK>
@@ -278,6 +288,13 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// threadIdx.x, read anew.
+__device__ __forceinline__ int fresh_tid() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile(
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -342,8 +359,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   if (warp < kTcWarps) {
     const int quarter = warp & 3, sgrp = warp >> 2;
     const uint32_t lanes = uint32_t(quarter * 32) << 16;
-    const int64_t to = tbase + 32 * quarter + lane;
-    const int64_t ic = to < ntarg ? to : ntarg - 1;
+    const int64_t it = tbase + 32 * quarter + lane;
+    const int64_t ic = it < ntarg ? it : ntarg - 1;
     const float fx = float(g.tx[ic] - cx), fy = float(g.ty[ic] - cy), fz = float(g.tz[ic] - cz);
     const float2 tx = make_float2(fx, fx), ty = make_float2(fy, fy), tz = make_float2(fz, fz);
     const int c0 = sgrp * NH;  // this thread's accumulator columns
@@ -355,7 +372,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     for (int n = 0; n < NH; ++n) sum2[kTwoSums ? n : 0] = 0.0;
     bool ok = true;
     auto drain = [&](int i) {  // tile i's accumulator into the registers
-      ok = tc_wait_warp(&sm.done, uint32_t(i) & 1u, fail);
+      ok = tc_wait_warp(&sm.done, uint32_t(i) & 1u, fail, c.spin);
       if (!ok) return;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       flush_add<N, NH, SPLIT>(tmem + lanes, c0, sum);
@@ -387,7 +404,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t a0 = acol + lanes + uint32_t(kTcPer * sgrp);
     for (int i = 0; i < ntiles; ++i) {
       const int s = i % ST;
-      ok = tc_wait_warp(&sm.full[s], uint32_t(i / ST) & 1u, fail);
+      ok = tc_wait_warp(&sm.full[s], uint32_t(i / ST) & 1u, fail, c.spin);
       if (!ok) break;
       const TcGeom& ge = sm.geom[s];
       float vr[kTcPer], vi[kTcPer];
@@ -433,9 +450,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       if (!kTwoSums && i > 0 && i % kTcFold == 0) fold();  // under this tile's MMAs
     }
     if (ok && ntiles > 0) drain(ntiles - 1);
+    // (the indices are formed anew: kept over the loop they would be spilled)
+    const int tid2 = fresh_tid(), c2 = (tid2 >> 7) * NH;
+    const int64_t to = int64_t(blockIdx.x) * kTcT + (tid2 & (kTcT - 1));
     if (ok && to < ntarg) {
-      // column c0 + n: real (< N) or imaginary part of density m0 + (c0 + n) % N
-      const int comp = c0 >= N ? 1 : 0, d0 = m0 + (c0 % N);
+      // column c2 + n: real (< N) or imaginary part of density m0 + (c2 + n) % N
+      const int comp = c2 >= N ? 1 : 0, d0 = int(blockIdx.z) * N + (c2 % N);
 #pragma unroll
       for (int n = 0; n < NH; ++n)
         if (d0 + n < nd) {
@@ -443,7 +463,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           partial[((size_t(blockIdx.y) * ntarg + to) * nd + d0 + n) * 2 + comp] =
               (1.0 + kTcLoss<N>) *
               (v + (kTwoSums ? sum2[kTwoSums ? n : 0]
-                             : double(sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid])));
+                             : double(sm.run[kTwoSums ? 0 : n][kTwoSums ? 0 : tid2])));
         }
     }
   } else if (warp == kTcWarps) {
@@ -490,7 +510,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const double g2 = gap * gap;
       const double gap2 = g2 + __shfl_down_sync(0xffffffffu, g2, 1) + __shfl_down_sync(0xffffffffu, g2, 2);
       if (i + 1 < ntiles) fetch(sg + kTcS);
-      if (i >= ST && !tc_wait_warp(&sm.empty[s], uint32_t(i / ST - 1) & 1u, fail)) break;
+      if (i >= ST && !tc_wait_warp(&sm.empty[s], uint32_t(i / ST - 1) & 1u, fail, c.spin)) break;
       TcGeom& ge = sm.geom[s];
 #pragma unroll
       for (int h = 0; h < H; ++h) {
@@ -518,18 +538,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
       issued = i + 1;
     }
-    if (*fail)  // the copies still in flight land before the CTA goes
-      for (int i = issued > ST ? issued - ST : 0; i < issued; ++i)
-        for (uint32_t r = 0; r < kTcSpin; ++r) {
-          uint32_t done;
-          asm volatile(
-              "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-              "selp.b32 %0, 1, 0, p;\n\t}\n"
-              : "=r"(done)
-              : "r"(smem_u32(&sm.full[i % ST])), "r"(uint32_t(i / ST) & 1u)
-              : "memory");
-          if (done) break;
-        }
+    // the copies still in flight land before the CTA goes: another role may give
+    // up after this one has left its loop
+    for (int i = issued > ST ? issued - ST : 0; i < issued; ++i)
+      for (uint32_t r = 0; r < kTcDrain; ++r)
+        if (tc_try(&sm.full[i % ST], uint32_t(i / ST) & 1u)) break;
   } else {
     // the whole warp walks the tiles, so that the operands of the MMAs stay
     // in uniform registers; one elected lane issues
@@ -538,8 +551,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     int issued = -1;
     for (int i = 0; i < ntiles; ++i) {
       const int s = i % ST;
-      if (!tc_wait_warp(&sm.full[s], uint32_t(i / ST) & 1u, fail)) break;
-      if (!tc_wait_warp(&sm.afull, uint32_t(i) & 1u, fail)) break;
+      if (!tc_wait_warp(&sm.full[s], uint32_t(i / ST) & 1u, fail, c.spin)) break;
+      if (!tc_wait_warp(&sm.afull, uint32_t(i) & 1u, fail, c.spin)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t bd = bdesc + uint64_t(uint32_t(s) * (kOpBytes >> 4));
       if (elect_one()) {
@@ -562,30 +575,29 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
           }
         }
+        tc_commit(&sm.empty[s]);  // (first: nobody waits for the last tile's)
         tc_commit(&sm.done);
-        tc_commit(&sm.empty[s]);
       }
       __syncwarp();
       issued = i;
     }
-    if (*fail && issued >= 0) {
-      // let the last committed MMAs finish before the tensor memory is freed
-      for (uint32_t r = 0; r < kTcSpin; ++r) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(smem_u32(&sm.done)), "r"(uint32_t(issued) & 1u)
-            : "memory");
-        if (done) break;
-      }
-    }
+    // the last committed MMAs finish before the tensor memory is freed
+    for (uint32_t r = 0; issued >= 0 && r < kTcDrain; ++r)
+      if (tc_try(&sm.done, uint32_t(issued) & 1u)) break;
   }
   __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (tid == 0 && *fail && err) atomicExch(err, 1 + int(blockIdx.x));
+  if (*fail) {
+    if (tid == 0 && err) atomicExch(err, 1 + int(blockIdx.x));
+    for (int q = fresh_tid(); q < kTcT * N; q += kTcThreads) {
+      const int64_t to = int64_t(blockIdx.x) * kTcT + q / N;
+      const int m = int(blockIdx.z) * N + q % N;
+      if (to < ntarg && m < nd)
+        reinterpret_cast<double2*>(partial)[(size_t(blockIdx.y) * ntarg + to) * nd + m] =
+            make_double2(CUDART_NAN, CUDART_NAN);
+    }
+  }
   if (warp == kTcWarps + 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(kTcTmemCols));
@@ -653,6 +665,7 @@ cudaError_t far_tc_go(const Geometry& g, const KParams& kp, const MatvecArgs& a,
   c.one = dup(1.0);
   c.mone = dup(-1.0);
   c.thr2 = float(kp.thresh * kp.thresh);
+  c.spin = a.tc_spin;
   kern<<<grid, kTcThreads, smem, st>>>(g, c, a.tc_ops, ntile, a.nd, a.partial, chunk, a.tc_err);
   return cudaGetLastError();
 }

@@ -25,6 +25,7 @@
 // an engine of its own (bie_set_oversample_engine) with its accuracy and its
 // time measured beside the CUDA-core kernel.
 #include <cuda_runtime.h>
+#include <math_constants.h>
 
 #include <atomic>
 #include <cstdint>
@@ -147,6 +148,12 @@ __global__ void __launch_bounds__(kOsThreads)
     }
   } else {
     if (tid == 0 && err) atomicExch(err, 1 + p);
+    // NaN rather than what the buffer held before
+    for (int q = tid; q < nf * nd; q += kOsThreads) {
+      const int64_t o = sdest ? sdest[os + q / nd] : os + q / nd;
+      sover[2 * (size_t(o) * nd + q % nd)] = CUDART_NAN_F;
+      sover[2 * (size_t(o) * nd + q % nd) + 1] = CUDART_NAN_F;
+    }
     for (int r = 0; r < 4; ++r)
       if (wait_phase(&bar, 0u)) break;
   }

@@ -887,6 +887,7 @@ int Plan::matvec(int precision, int nd, const double* d_sigma, double* d_pot, cu
   a.weff_f32 = precision == 1;
   a.ab = precision == 1 ? (const void*)ab32_.p : (const void*)ab64_.p;
   a.tc_err = tc_err_.p;
+  a.tc_spin = tc_spin;
   a.tc_ops = tc_ops_.p;
   if (timing) BIE_CUDA(cudaEventRecord(ev_[0], st));
   if (nd > 1)

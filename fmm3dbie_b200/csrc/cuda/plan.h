@@ -251,8 +251,11 @@ class Plan : public Operator {
   // Pins the far-field shape and chunk count of (precision, nd) instead of
   // tuning it; variant as dev::far_variants().
   int set_far_config(int precision, int nd, int variant, int nchunks);
-  // Nonzero once a tensor-core far-field launch timed out waiting for its MMAs.
+  // Nonzero once a tensor-core far-field launch timed out waiting for its MMAs
+  // (its potentials are NaN).
   int tc_error() const;
+  // polls that a wait of the tensor-core far field may take
+  uint32_t tc_spin = dev::kTcSpin;
   int* tc_err_ptr() { return tc_err_.p; }
   // makes st wait for W_eff (a no-op unless the plan was built with async_weff)
   int wait_weff(cudaStream_t st);

@@ -82,6 +82,12 @@ class Plan:
         L.check(L.lib().bie_plan_get_far(self._h, iprec, nd, L.ptr(out)), "bie_plan_get_far")
         return tuple(int(v) for v in out)
 
+    def set_tc_wait(self, polls: int = -1):
+        """Polls that a wait of the tensor-core far field may take (-1: the
+        default).  A launch that runs out of them leaves NaN potentials and
+        sets get_far's flag."""
+        L.check(L.lib().bie_plan_set_tc_wait(self._h, polls), "bie_plan_set_tc_wait")
+
     def set_far_method(self, iprec: int, method: int, theta: float = 0.0, p: int = 0,
                        leaf_t: int = 0, leaf_s: int = 0):
         """Far field of precision iprec: 0 direct sum, 1 hierarchical

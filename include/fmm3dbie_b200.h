@@ -381,11 +381,16 @@ int bie_plan_oversample(void* plan, int64_t engine, int64_t nd, const double* si
 /* Far-field shape of (iprec, nd): bie_plan_set_far pins it (variant 0-2:
  * CUDA-core block shapes; 3-4: matrix-instruction kernels of the Helmholtz
  * multi-density path, 16/32 or 64 densities per CTA: tensor cores in FP32 for
- * nd >= 2, FP64 matrix instructions for nd > 8; nchunks source chunks) instead of the autotuner's choice; bie_plan_get_far returns the
- * variant, the chunk count and a nonzero flag if a tensor-core launch timed
- * out waiting for its MMAs.  No reference counterpart. */
+ * nd >= 2, FP64 matrix instructions for nd > 8; nchunks source chunks)
+ * instead of the autotuner's choice; bie_plan_get_far returns the variant, the
+ * chunk count and a nonzero flag if a tensor-core launch timed out waiting for
+ * its copies or MMAs.  The potentials of such a launch are NaN, and a solve
+ * that meets them returns BIE_BREAKDOWN.  bie_plan_set_tc_wait: polls that
+ * a wait of the tensor-core far field may take before it gives up (< 0: the
+ * default; 0: every wait gives up).  No reference counterpart. */
 int bie_plan_set_far(void* plan, int64_t iprec, int64_t nd, int64_t variant, int64_t nchunks);
 int bie_plan_get_far(void* plan, int64_t iprec, int64_t nd, int64_t* out);
+int bie_plan_set_tc_wait(void* plan, int64_t polls);
 /* Far-field method of precision iprec, replacing the lfmm3d / hfmm3d calls
  * of lpcomp_*_addsub (lap_comb_dir.f90:1094, helm_comb_dir.f:1117):
  * method 0 = direct sum over all target-source pairs, 1 = hierarchical
