@@ -4,6 +4,7 @@
 // Givens rotations and stopping test; all systems share every launch.
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -34,17 +35,36 @@ std::vector<double> interleave(const std::vector<cdouble>& v) {
   return o;
 }
 
-// Waits until a kernel in stream st has written *word >= least; a stream that
-// ends without it (an error) ends the wait.  The stop flag of an iteration by
-// a copy and a stream synchronisation took 26 us from the Givens step to the
-// next matvec's first kernel, this 8.
-cudaError_t poll_word(const volatile int64_t* word, int64_t least, cudaStream_t st) {
-  for (int spin = 1; *word < least; ++spin) {
-    if (spin % 4096) continue;
-    const cudaError_t e = cudaStreamQuery(st);
-    if (e == cudaErrorNotReady) continue;
+// How long a wait for a solver's stop flag polls it before it leaves the wait to
+// the driver: the flag by a copy and a stream synchronisation took 26 us from
+// the Givens step to the next matvec's first kernel, polled 8, which counts
+// where a product is short.  A process that asked for blocking or yielding waits
+// gets those from the start.
+std::chrono::microseconds poll_time() {
+  unsigned flags = 0;
+  if (cudaGetDeviceFlags(&flags) != cudaSuccess) {
+    cudaGetLastError();
+    flags = 0;
+  }
+  const unsigned mode = flags & cudaDeviceScheduleMask;
+  const bool spins = mode == cudaDeviceScheduleAuto || mode == cudaDeviceScheduleSpin;
+  return std::chrono::microseconds(spins ? 1000 : 0);
+}
+
+// Waits until a kernel in stream st has written *word >= least: polls for at most
+// `poll`, then waits for the stream the way the driver does; a stream that ends
+// without it (an error) ends the wait.
+cudaError_t poll_word(const volatile int64_t* word, int64_t least, cudaStream_t st,
+                      std::chrono::microseconds poll) {
+  const auto t0 = std::chrono::steady_clock::now();
+  while (poll.count() > 0 && *word < least) {
+    for (int spin = 0; spin < 64 && *word < least; ++spin) __builtin_ia32_pause();
+    if (std::chrono::steady_clock::now() - t0 > poll) break;
+  }
+  if (*word < least) {
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
-    return *word < least ? cudaErrorUnknown : cudaSuccess;
+    if (*word < least) return cudaErrorUnknown;
   }
   std::atomic_thread_fence(std::memory_order_acquire);
   return cudaSuccess;
@@ -161,10 +181,12 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
   BIE_CUDA(ws.brk.alloc(nsys));
   // a single system's stop flag is polled, those of several are copied
   int64_t* status = nullptr;
+  std::chrono::microseconds poll{0};
   if (nsys == 1) {
     BIE_CUDA(ws.status.alloc());
     status = ws.status.p;
     *status = -1;
+    poll = poll_time();
   }
   double* d_H = ws.ls.p;
   double* d_cs = d_H + nH;
@@ -180,7 +202,7 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
   // stop flags after `step` iterations (0: the start)
   auto read_done = [&](int64_t step) -> int {
     if (status) {
-      BIE_CUDA(poll_word(status, 2 * step, st));
+      BIE_CUDA(poll_word(status, 2 * step, st, poll));
       if (*static_cast<volatile int64_t*>(status) & 1) done[0] = step > 0 ? step : -1;
       return kOk;
     }
