@@ -751,7 +751,7 @@ int Plan::set_far_config(int precision, int nd, int variant, int nchunks) {
   c.variant = variant;
   c.nchunks = nchunks;
   far_cfg_[{precision, nd}] = c;
-  return ensure_workspace(precision, nd, nchunks);
+  return ensure_workspace(precision, nd, c);
 }
 
 int Plan::tc_error() const {
@@ -777,33 +777,54 @@ cudaError_t Plan::launch_far_stage(const dev::MatvecArgs& a, cudaStream_t st) {
   return a.nd > 1 ? dev::launch_far_md(g, kp, a, st) : dev::launch_far(g, kp, a, st);
 }
 
-int Plan::ensure_workspace(int precision, int nd, int nchunks) {
+bool Plan::uses_tc_ops(int precision, int nd, const FarConfig& c) const {
+  return nd > 1 && precision == 1 && far_method_[1] == 0 &&
+         dev::far_tc_group(c.variant, nd, precision, kind) > 0;
+}
+
+int Plan::ensure_workspace(int precision, int nd, const FarConfig& c) {
   const size_t sreals = size_t(nptso) * nd * (cplx ? 4 : 2);
   BIE_CUDA(str_.alloc(sreals * sizeof(double)));
-  BIE_CUDA(partial_.alloc(std::max<size_t>(1, size_t(nchunks) * ntarg * nd * (cplx ? 2 : 1))));
-  if (far_method_[precision & 1] == 0)
+  BIE_CUDA(partial_.alloc(std::max<size_t>(1, size_t(c.nchunks) * ntarg * nd * (cplx ? 2 : 1))));
+  // (0.25 to 4 KB a source: only for the shapes that read it)
+  if (uses_tc_ops(precision, nd, c))
     BIE_CUDA(tc_ops_.alloc(dev::far_tc_operand_floats(nd, precision, kind, nptso)));
   return kOk;
 }
 
 int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, FarConfig& best) {
   const FarKey key{device, kind, kp.ki != 0.0 ? 1 : 0, precision, nd, ntarg, nptso};
+  // room for the tensor-core shapes' operand; without it the others remain
+  auto tc_room = [&] {
+    if (tc_ops_.alloc(dev::far_tc_operand_floats(nd, precision, kind, nptso)) == cudaSuccess)
+      return true;
+    cudaGetLastError();
+    return false;
+  };
+  bool known = false;
   {
     std::lock_guard<std::mutex> lk(g_far_mu);
     auto it = g_far_cache.find(key);
     if (it != g_far_cache.end()) {
+      known = true;
       best = it->second;
-      return kOk;
     }
   }
+  if (known && (!uses_tc_ops(precision, nd, best) || tc_room())) return kOk;
+  bool all_shapes = true;
   best = far_config(precision, nd);
   const bool fixed = std::getenv("BIE_FAR_VARIANT") || std::getenv("BIE_FAR_WAVES") ||
                      env_int("BIE_AUTOTUNE", 1) == 0;
   if (!fixed && ntarg > 0) {
     std::vector<FarConfig> cand;
     const int md = nd > 1;
+    const bool tc = precision == 0 || tc_room();
     for (int v = 0; v < dev::far_variants(); ++v) {
       if (v == dev::kFarSmall && !dev::far_small_fits(ntarg, nd)) continue;
+      if (!tc && md && dev::far_tc_group(v, nd, precision, kind) > 0) {
+        all_shapes = false;
+        continue;
+      }
       const int bps = dev::far_blocks_per_sm(kp, precision, v, md, nd);
       if (bps <= 0) continue;
       for (double waves : {1.0, 2.0, 4.0, 8.0}) {
@@ -818,11 +839,12 @@ int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, F
         if (!dup) cand.push_back(c);
       }
     }
-    int maxch = 1;
-    for (const auto& c : cand) maxch = std::max(maxch, c.nchunks);
-    int ier = ensure_workspace(precision, nd, maxch);
+    FarConfig most;
+    for (const auto& c : cand) most.nchunks = std::max(most.nchunks, c.nchunks);
+    int ier = ensure_workspace(precision, nd, most);
     if (ier) return ier;
     a.partial = partial_.p;
+    a.tc_ops = tc_ops_.p;
     cudaEvent_t e0, e1;
     BIE_CUDA(cudaEventCreate(&e0));
     BIE_CUDA(cudaEventCreate(&e1));
@@ -849,9 +871,15 @@ int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, F
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    // the operand goes back unless a shape of this plan reads it
+    bool used = uses_tc_ops(precision, nd, best);
+    for (const auto& f : far_cfg_) used |= uses_tc_ops(f.first.first, f.first.second, f.second);
+    if (!used) tc_ops_.release();
   }
-  std::lock_guard<std::mutex> lk(g_far_mu);
-  g_far_cache[key] = best;
+  if (all_shapes) {
+    std::lock_guard<std::mutex> lk(g_far_mu);
+    g_far_cache[key] = best;
+  }
   return kOk;
 }
 
@@ -872,7 +900,7 @@ int Plan::matvec(int precision, int nd, const double* d_sigma, double* d_pot, cu
   }
   if (far_method_[precision & 1] == 1) return matvec_tree(precision, nd, d_sigma, d_pot, st);
   FarConfig fc = far_config(precision, nd);
-  int ier = ensure_workspace(precision, nd, fc.nchunks);
+  int ier = ensure_workspace(precision, nd, fc);
   if (ier) return ier;
   dev::MatvecArgs a;
   a.precision = precision;
@@ -898,11 +926,12 @@ int Plan::matvec(int precision, int nd, const double* d_sigma, double* d_pot, cu
     ier = tune_far(precision, nd, a, st, fc);
     if (ier) return ier;
     far_cfg_[{precision, nd}] = fc;
-    ier = ensure_workspace(precision, nd, fc.nchunks);
+    ier = ensure_workspace(precision, nd, fc);
     if (ier) return ier;
     a.nchunks = fc.nchunks;
     a.far_variant = fc.variant;
     a.partial = partial_.p;
+    a.tc_ops = tc_ops_.p;
     if (timing) BIE_CUDA(cudaEventRecord(ev_[1], st));
   } else if (timing) {
     BIE_CUDA(cudaEventRecord(ev_[1], st));
@@ -929,7 +958,7 @@ int Plan::matvec(int precision, int nd, const double* d_sigma, double* d_pot, cu
 int Plan::matvec_tree(int precision, int nd, const double* d_sigma, double* d_pot,
                       cudaStream_t st) {
   TreeFar& T = *tree_[precision];
-  int ier = ensure_workspace(precision, nd, 1);
+  int ier = ensure_workspace(precision, nd, FarConfig());
   if (ier) return ier;
   dev::MatvecArgs a;
   a.precision = precision;

@@ -288,7 +288,9 @@ class Plan : public Operator {
   StageTimes times;
 
  private:
-  int ensure_workspace(int precision, int nd, int nchunks);
+  // the buffers that a product with shape c needs
+  int ensure_workspace(int precision, int nd, const FarConfig& c);
+  bool uses_tc_ops(int precision, int nd, const FarConfig& c) const;
   int refold32(const double* tcen, cudaStream_t st);
   int matvec_tree(int precision, int nd, const double* d_sigma, double* d_pot, cudaStream_t st);
   int tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, FarConfig& out);
@@ -301,8 +303,8 @@ class Plan : public Operator {
   DBuf<int64_t> cmoff_, row_ptr_, wofs_;
   DBuf<double> weff64_;
   DBuf<float> weff32_;
-  DBuf<float> tc_ops_;  // its density operand
-  DBuf<int> tc_err_;  // timeout flag of the tensor-core far field
+  DBuf<float> tc_ops_;  // density operand of the tensor-core far field
+  DBuf<int> tc_err_;    // its timeout flag
   std::unique_ptr<TreeFar> tree_[2];
   int far_method_[2] = {0, 0};
   DBuf<char> str_;
