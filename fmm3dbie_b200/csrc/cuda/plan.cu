@@ -67,12 +67,29 @@ int cached_interp_matrix(int ip, int no, int nf, const std::vector<double>*& m) 
   return 0;
 }
 
-// Pinned staging for the arrays a plan build assembles on the host, shared by
-// the builds of the process one at a time.  It is allocated (its pages
-// faulted in) once and grown when a larger plan comes, so the uploads out of
-// it are asynchronous and a build pays no page faults.  A build that finds it
-// in use by another thread, or needs more than kMaxPinned bytes, stages in
-// pageable memory instead.  The destructor waits for the copies out of it.
+// A pinned buffer of the process, used by one thread at a time.  It is allocated
+// (its pages faulted in) once and grown when a larger user comes.
+struct PinnedPool {
+  std::mutex mu;
+  char* p = nullptr;
+  size_t cap = 0;
+};
+// Never destroyed: builds may run during exit.
+PinnedPool& build_pool() {
+  static PinnedPool* p = new PinnedPool;
+  return *p;
+}
+PinnedPool& download_pool() {
+  static PinnedPool* p = new PinnedPool;
+  return *p;
+}
+
+// Pinned staging for the arrays a plan build assembles on the host and (from a
+// pool of their own, so that neither waits for the other) for results on their
+// way to the host: the copies are asynchronous and pay no page faults.  A build
+// that finds its pool in use by another thread, or needs more than kMaxPinned
+// bytes, stages in pageable memory instead; without `pageable` there is no
+// buffer then (pinned() is false).  The destructor waits for the copies.
 class HostStaging {
  public:
   static constexpr size_t kMaxPinned = size_t(256) << 20;
@@ -80,8 +97,8 @@ class HostStaging {
   static size_t bytes(size_t n) {
     return (n * sizeof(T) + 63) / 64 * 64;
   }
-  explicit HostStaging(size_t n) : cap_(n) {
-    Pool& pl = pool();
+  explicit HostStaging(size_t n, PinnedPool& pl = build_pool(), bool pageable = true)
+      : pool_(pl), cap_(n) {
     if (n <= kMaxPinned && pl.mu.try_lock()) {
       locked_ = true;
       if (pl.cap < n) {
@@ -99,18 +116,19 @@ class HostStaging {
       }
       base_ = pl.p;
     }
-    if (!base_) {
+    pinned_ = base_ != nullptr;
+    if (!base_ && pageable) {
       heap_.reset(new char[n + 64]);
       base_ = heap_.get() + (64 - reinterpret_cast<uintptr_t>(heap_.get()) % 64) % 64;
     }
   }
   ~HostStaging() {
     if (st_set_) cudaStreamSynchronize(st_);
-    if (locked_) pool().mu.unlock();
+    if (locked_) pool_.mu.unlock();
   }
   HostStaging(const HostStaging&) = delete;
   HostStaging& operator=(const HostStaging&) = delete;
-  bool pinned() const { return !heap_; }
+  bool pinned() const { return pinned_; }
   // the stream that the uploads out of the buffer are issued on
   void copies_on(cudaStream_t st) {
     st_ = st;
@@ -126,18 +144,10 @@ class HostStaging {
   }
 
  private:
-  struct Pool {
-    std::mutex mu;
-    char* p = nullptr;
-    size_t cap = 0;
-  };
-  static Pool& pool() {
-    static Pool* p = new Pool;  // never destroyed: builds may run during exit
-    return *p;
-  }
+  PinnedPool& pool_;
   char* base_ = nullptr;
   size_t cap_ = 0, off_ = 0;
-  bool locked_ = false, st_set_ = false;
+  bool locked_ = false, pinned_ = false, st_set_ = false;
   cudaStream_t st_ = nullptr;
   std::unique_ptr<char[]> heap_;
 };
@@ -165,7 +175,7 @@ cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t 
     const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
     return e != cudaSuccess ? e : cudaStreamSynchronize(st);
   }
-  HostStaging stage(slots * piece);
+  HostStaging stage(slots * piece, download_pool(), false);
   if (!stage.pinned()) {  // in use by another thread
     const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
     return e != cudaSuccess ? e : cudaStreamSynchronize(st);

@@ -63,9 +63,9 @@ struct AllocStreamScope {
 // a fresh allocation are then in place when the result arrives.
 void prefault(void* p, size_t bytes);
 // Copies device memory to a host buffer and waits for it.  Pageable buffers of
-// several MB go through the process's pinned staging buffer in pieces that
+// several MB go through a pinned staging buffer of the process in pieces that
 // several threads move on while the next ones arrive (the driver's own
-// pageable copy: about 5 GB/s into fresh pages).
+// pageable copy, which a second thread gets: about 5 GB/s into fresh pages).
 cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
 template <class T>
