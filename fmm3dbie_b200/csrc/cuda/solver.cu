@@ -253,9 +253,18 @@ int gmres(Operator& P, int precision, int rres_precision, int nd, const cdouble*
     gv.status = status;
     double* w = ws.w.p;
     double* pt = ws.partial.p;
+    bool orth_done = false;
     if (nsys == 1 && dev::orth_cluster_fits(n, m)) {
-      BIE_CUDA(dev::launch_orth_cluster(V, ldv, m, w, wts, n, cplx, vnext, gv, st));
-    } else {
+      const cudaError_t e = dev::launch_orth_cluster(V, ldv, m, w, wts, n, cplx, vnext, gv, st);
+      // no room for a cluster (a device shared by partition): the kernels below
+      if (e == cudaErrorInvalidClusterSize || e == cudaErrorLaunchOutOfResources) {
+        cudaGetLastError();
+      } else {
+        BIE_CUDA(e);
+        orth_done = true;
+      }
+    }
+    if (!orth_done) {
       BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h1, nullptr, 0, nullptr, nullptr, st));
       BIE_CUDA(dev::launch_orth(V, ldv, m, w, wts, nd, cplx, sg, pt, d_h2, d_h1, m, V, nullptr, st));
       BIE_CUDA(dev::launch_orth(w, ldv, 1, w, wts, nd, cplx, sg, pt, d_nrm, d_h2, m, V, &gv, st));
