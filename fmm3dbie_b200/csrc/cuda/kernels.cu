@@ -2852,7 +2852,9 @@ cudaError_t launch_combine(const Geometry& g, const Near& nr, const KParams& kp,
   };
   const float* wf = static_cast<const float*>(a.weff);
   const double* wd = static_cast<const double*>(a.weff);
-  if (kp.kind == 1 && combine_mode(a.nd) == kCombineWide &&
+  // (the wide form takes complex values at any 8-byte boundary)
+  const bool pairs = ((reinterpret_cast<uintptr_t>(a.sigma) | reinterpret_cast<uintptr_t>(a.pot)) & 15) == 0;
+  if (kp.kind == 1 && combine_mode(a.nd) == kCombineWide && pairs &&
       combine_mma_warps(g.ntarg, a.nd) >= kCombineMmaWarps) {
     if (a.weff_f32)
       launch_combine_mma(g, nr, wf, a, st);
