@@ -153,7 +153,20 @@ class HostStaging {
 };
 }  // namespace
 
+namespace {
+// What CUDA knows p as; plain host memory is cudaMemoryTypeUnregistered.
+cudaMemoryType memory_type(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return cudaMemoryTypeUnregistered;
+  }
+  return at.type;
+}
+}  // namespace
+
 void prefault(void* p, size_t bytes) {
+  if (bytes == 0 || memory_type(p) != cudaMemoryTypeUnregistered) return;
   constexpr size_t page = 4096;
   char* c = static_cast<char*>(p);
   const int64_t n = int64_t((bytes + page - 1) / page);
@@ -167,10 +180,7 @@ void prefault(void* p, size_t bytes) {
 cudaError_t copy_to_host(void* dst, const void* src, size_t bytes, cudaStream_t st) {
   constexpr size_t piece = size_t(4) << 20;
   constexpr int slots = 4;
-  cudaPointerAttributes at{};
-  const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
-                      at.type != cudaMemoryTypeUnregistered;
-  if (!pinned) cudaGetLastError();
+  const bool pinned = memory_type(dst) != cudaMemoryTypeUnregistered;
   if (pinned || bytes < 2 * piece) {
     const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
     return e != cudaSuccess ? e : cudaStreamSynchronize(st);

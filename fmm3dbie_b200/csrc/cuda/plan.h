@@ -58,9 +58,10 @@ struct AllocStreamScope {
   AllocStreamScope& operator=(const AllocStreamScope&) = delete;
 };
 
-// Touches every page of a host buffer that a running device computation will
-// fill, with several threads and without changing its contents: the pages of
-// a fresh allocation are then in place when the result arrives.
+// Touches every page of a pageable host buffer that a running device computation
+// will fill, with several threads and without changing its contents: the pages
+// of a fresh allocation are then in place when the result arrives.  (Other
+// memory is left alone: the host cannot read device memory.)
 void prefault(void* p, size_t bytes);
 // Copies device memory to a host buffer and waits for it.  Pageable buffers of
 // several MB go through a pinned staging buffer of the process in pieces that
