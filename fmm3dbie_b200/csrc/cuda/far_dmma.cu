@@ -13,11 +13,12 @@
 // in FP64 accumulators kept in registers over the whole chunk.
 //
 // The CUDA-core kernel (far_md_kernel) holds 16 densities a thread and so
-// evaluates every kernel value four times at 64 densities (416 operations a
-// pair against 296 here), with one instruction per multiply-add; a matrix
-// instruction is 256 of them.  Both are bound by the FP64 pipe.  36,504 targets
-// x 77,974 sources: 64 densities 86.3 -> 50.8 ms (46 ms at the pipe's peak), 24
-// densities 44.4 -> 29.2, 16 densities 22.8 -> 18.8.
+// evaluates every kernel value four times at 64 densities (424 operations a
+// pair against 298 here), with one instruction per multiply-add; a matrix
+// instruction is 256 of them.  Both are bound by the FP64 pipe (here 90 % busy,
+// 77 % of it with matrix instructions).  36,504 targets x 77,910 sources: 64
+// densities 86.3 -> 52.5 ms (47 ms at the pipe's peak), 24 densities 44.4 ->
+// 30.2, 16 densities 22.8 -> 19.1.
 #include <cuda_runtime.h>
 
 #include <cstdint>

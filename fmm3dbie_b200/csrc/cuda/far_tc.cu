@@ -26,9 +26,11 @@
 // 18 warps per CTA, ordered only by mbarriers:
 //   warps 0-15  kernel values (warp w: targets 32 (w % 4) .. + 31, one per
 //               lane, sources 16 (w / 4) .. + 15 of the tile, two per packed
-//               instruction) with the FP32 pair arithmetic and block centring
-//               of the CUDA-core kernels, so that the error-matched W_eff32
-//               fold still cancels their near-pair values; and the sums: each
+//               instruction) with the FP32 coordinates, block centring and
+//               kernel of the CUDA-core kernels, whose rounding of a close
+//               pair the error-matched W_eff32 fold cancels (the weight goes to
+//               the density, so the values differ from theirs by roundings of
+//               their own size); and the sums: each
 //               thread adds N / 2 columns of its target into FP32 registers
 //               after every tile and every kTcFold tiles into FP64 ones (64
 //               densities: into FP32 sums in shared memory, compensated);
@@ -39,13 +41,16 @@
 //               instead of 5.7 ms at 16 densities).
 // While the tensor core works on a tile the SIMT warps evaluate the next.
 //
-// Measured (matvec of a 36,504-node surface with 77,974 oversampled nodes,
-// B200): 64 densities 17.3 -> 7.7 ms, 32: 15.5 -> 5.7, 16: 11.9 (CUDA cores)
-// -> 5.3, 4: 6.0 (CUDA cores) -> 5.0, against FP64 6.3e-7 (9.2e-7 before) at
-// 64 densities and 5.0e-7 (5.0e-7) at 16.  What bounds it: at 64 densities
-// the 48 MMAs of a tile (about 104 cycles each; 64 would be the tensor peak),
-// below that the kernel values with the operand splits (about 25 instructions
-// a pair; evaluation alone takes 3.4 of the 4.5 ms at 16 densities).
+// Measured (matvec of a 36,504-node surface with 77,910 oversampled nodes,
+// B200, against the kernel with serial stages or, up to 16 densities, the CUDA
+// cores): 64 densities 17.3 -> 7.3 ms, 32: 15.5 -> 5.4, 16: 11.9 -> 5.0, 8: 8.4
+// -> 5.0; at 4 both take 4.9 and the tuner keeps the CUDA cores.  Distance from
+// the FP64 product there (k = 2, mean over plane waves): 64 densities 7.5e-7 ->
+// 1.5e-7, 32: 7.5e-7 -> 1.3e-7, 16: 1.5e-7 -> 1.4e-7.  What bounds it: at 64
+// densities the 48 MMAs of a tile (about 104 cycles each, 6.0 of the 7.3 ms; 64
+// cycles would be the nominal rate) and the drain and the store of A between
+// them, below that the kernel values with the operand splits (about 25
+// instructions a pair; evaluation alone takes 3.4 of the 4.8 ms at 16).
 //
 // Completion waits are bounded (MatvecArgs::tc_spin polls); on timeout the
 // kernel records the CTA in *err, every role leaves, the copies and MMAs in
@@ -79,8 +84,8 @@ constexpr uint32_t kTcTmemCols = 512;
 // Parts a tile's sources are split into for N densities: each part has its own
 // two accumulators (Kr and Ki) of 2 N columns, so that an accumulator rounds
 // at full size in 8 / parts hi*hi steps.  As many as tensor memory holds at 16
-// densities (against FP64 on a 3,750-node sphere: 1.1e-7 with 4 parts, 2.4e-7
-// with 1; the CUDA-core kernel 1.14e-7).
+// densities (against FP64 on a 3,750-node sphere, without kTcLoss: 1.1e-7 with 4
+// parts, 2.4e-7 with 1; the CUDA-core kernel 1.14e-7).
 template <int N>
 constexpr int kTcSplit = N == 64 ? 1 : (N == 32 ? 2 : 4);
 
@@ -162,8 +167,6 @@ __device__ __forceinline__ void tc_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Kernel values K = alpha G + beta dG/dn of one target against two sources
-// (lane .x and lane .y): per lane the operations of pair_helm.
 // Constants of the kernel values, each twice (the two lanes); a kernel
 // parameter, so that they stay in the constant bank.
 struct TcConst {
@@ -172,6 +175,9 @@ struct TcConst {
   uint32_t spin;  // polls of a wait
 };
 
+// Kernel values K = alpha G + beta dG/dn of one target against two sources
+// (lane .x and lane .y): the operations of pair_helm on the kernel's own constants
+// in the place of a source's strengths.
 template <bool CHECK, bool CK>
 __device__ __forceinline__ void tc_pair(const float2 tx, const float2 ty, const float2 tz,
                                         const float2 msx, const float2 msy, const float2 msz,

@@ -415,9 +415,9 @@ __global__ void __launch_bounds__(NT, (kFarMinBlocks<R, NT>)) far_kernel(Geometr
 // shapes above give a thread 1 to 8 targets and a whole tile, so a problem of
 // about a thousand targets leaves most of the chip without a warp and each
 // warp with a serial chain over 128 sources a tile.  864 targets x 2,646
-// sources (with about 5 us of launch and event time): Helmholtz FP64 21.6 ->
-// 15.8 us, FP32 17.4 -> 9.7, Laplace FP64 13.4 -> 11.1, FP32 13.0 -> 9.1; from
-// 5,400 targets on the other shapes are faster (they read each source for 2 to
+// sources (four launches back to back, each side's best chunk count): Helmholtz
+// FP64 21.2 -> 14.6 us, FP32 15.1 -> 6.9, Laplace FP64 11.0 -> 9.0, FP32 11.0 ->
+// 6.4; from 5,400 targets on the other shapes are faster (they read each source for 2 to
 // 8 targets).  The target's sums of the four warps are added in order at the
 // end.
 constexpr int kSmallTargets = 32, kSmallThreads = 128;

@@ -391,11 +391,13 @@ struct RawSource {
 // Near lists of a leaf's targets (PROXYT = false) or proxy potentials of 128
 // of a node's proxies (PROXYT = true).  One barrier per tile: the tile is
 // double-buffered, and the next one's sources are already in registers.
-// FP32 is bound by the XU pipe (3 MUFU operations a pair; 68 % busy in the
-// leaves, 80 % in the proxies), FP64 by the FP64 pipe.  Far field of 146,016
-// Helmholtz nodes (320,312 sources): FP32 10.9 -> 9.6 ms, FP64 49.6 -> 42.3
-// (with pair.cuh's FP64 pair); 207,576 Laplace nodes: 6.9 -> 4.9 and 23.8 ->
-// 21.2.  Before, one source at a time in one buffer, the downward pass in
+// FP32 is bound by the XU pipe (3 MUFU operations a pair; 64 % busy in the
+// leaves of a 55,296-node surface, FMA 55 %) and the barriers of short entries,
+// FP64 by the FP64 pipe (65 % there) and the same.  Whole far field of 146,016
+// Helmholtz nodes (320,312 sources), with pair.cuh's FP64 pair and the upward
+// pass above: FP32 10.9 -> 9.3 ms, FP64 49.6 -> 42.6; 207,576 Laplace nodes:
+// 6.9 -> 4.5 and 23.8 -> 20.3.  Before, one source at a time in one buffer, the
+// downward pass in
 // the same kernel, and a quarter to half of a leaf's warps idle.
 template <int KIND, typename R, bool CK, bool PROXYT>
 __global__ void __launch_bounds__(kEvBlock<PROXYT>, (kEvMinBlocks<KIND, R, PROXYT>))
