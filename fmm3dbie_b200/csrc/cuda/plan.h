@@ -139,22 +139,21 @@ struct PlanSpec {
   bool async_weff = false;
 };
 
-// One word of pinned host memory that kernels write and the host polls.
+// One word of pinned host memory that kernels write and the host polls, from
+// pages that the process keeps (a pinned allocation of its own took a new
+// plan's first solve 1.5 to 4 ms): taken by alloc, given back at the end.
+// Whoever destroys it has waited for the kernels that write it.
 struct HostWord {
   int64_t* p = nullptr;
   HostWord() = default;
   HostWord(const HostWord&) = delete;
   HostWord& operator=(const HostWord&) = delete;
-  ~HostWord() {
-    if (p) cudaFreeHost(p);
-  }
-  cudaError_t alloc() {
-    return p ? cudaSuccess
-             : cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(int64_t), cudaHostAllocPortable);
-  }
+  ~HostWord();
+  cudaError_t alloc();
 };
 
 struct GmresWorkspace {
+  HostWord status;  // of a single system's last Givens step (first: freed after the buffers)
   DBuf<double> V, w, partial, dots, coef, scale;
   // least squares on the device: Hessenberg columns, rotations, residual
   // vector, norms, tolerances and error history per system
@@ -162,7 +161,6 @@ struct GmresWorkspace {
   DBuf<int64_t> done;
   DBuf<int> brk;
   DBuf<double> zc;  // Krylov-basis coefficients of the residual vector
-  HostWord status;  // of a single system's last Givens step
 };
 
 struct MixedWorkspace {

@@ -7,6 +7,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -71,6 +72,44 @@ cudaError_t poll_word(const volatile int64_t* word, int64_t least, cudaStream_t 
 }
 
 }  // namespace
+
+namespace {
+// Free words, one cache line each, of pinned pages that are never returned: as
+// many as the process ever had operators solving at a time (64 a page).
+struct WordPool {
+  static constexpr size_t kLine = 64, kPage = 4096;
+  std::mutex mu;
+  std::vector<int64_t*> free;
+};
+// Never destroyed: operators may be released during exit.
+WordPool& word_pool() {
+  static WordPool* p = new WordPool;
+  return *p;
+}
+}  // namespace
+
+cudaError_t HostWord::alloc() {
+  if (p) return cudaSuccess;
+  WordPool& pl = word_pool();
+  std::lock_guard<std::mutex> lk(pl.mu);
+  if (pl.free.empty()) {
+    void* q = nullptr;
+    const cudaError_t e = cudaHostAlloc(&q, WordPool::kPage, cudaHostAllocPortable);
+    if (e != cudaSuccess) return e;
+    for (size_t o = 0; o < WordPool::kPage; o += WordPool::kLine)
+      pl.free.push_back(reinterpret_cast<int64_t*>(static_cast<char*>(q) + o));
+  }
+  p = pl.free.back();
+  pl.free.pop_back();
+  return cudaSuccess;
+}
+
+HostWord::~HostWord() {
+  if (!p) return;
+  WordPool& pl = word_pool();
+  std::lock_guard<std::mutex> lk(pl.mu);
+  pl.free.push_back(p);
+}
 
 int Operator::init_segments(cudaStream_t st) {
   const int ns = nseg();
