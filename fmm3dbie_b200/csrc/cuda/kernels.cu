@@ -2947,10 +2947,16 @@ cudaError_t launch_reduce_partials(int kind, const double* partial, int nchunks,
   return cudaGetLastError();
 }
 
-// Chunk sums times outputs that the last block of orth_kernel takes itself
-// (16 bytes each, read by one SM: 128 KB, about 2 us, the price of the
-// launch it saves); larger reductions go to mdot_final_kernel.
-constexpr int64_t kFusedReduce = 8192;
+// What the last block of orth_kernel takes itself: at most 8,192 chunk sums (16
+// bytes each, read by one SM: 128 KB, about 2 us, the price of the launch it
+// saves) of at most 32 outputs (vectors times systems).  A warp takes one output
+// at a time, about half a microsecond of latency each, and one system's Givens
+// step; larger reductions go to mdot_final_kernel and gmres_givens_kernel, which
+// spread over the chip.  Solves of 864 complex nodes, in microseconds, no limit on
+// the outputs / 256 / 64 / 32 / 9 launches an iteration: 4 systems 2577 / 2571 /
+// 2499 / 2494 / 3431, 16: 4542 / 4181 / 3993 / 3989 / 5150, 40: 7998 / 7495 / 7378 /
+// 7036 / 7558; 40 real systems 3142 / 2778 / 2676 / 2556 / 2559.
+constexpr int64_t kFusedReduce = 8192, kFusedOutputs = 32;
 
 cudaError_t launch_orth(const double* V, int64_t ldv, int m, double* w, const double* wts, int nd,
                         int cplx, const Segs& sg, double* partial, double* out,
@@ -2960,7 +2966,8 @@ cudaError_t launch_orth(const double* V, int64_t ldv, int m, double* w, const do
   if (nd < 1 || nd > 256) return cudaErrorInvalidValue;
   const int threads = (256 / nd) * nd;
   // the fused tail works in whole warps
-  const bool fused = int64_t(m) * nd * sg.nchunk <= kFusedReduce && sg.ticket && threads >= 32;
+  const bool fused = int64_t(m) * nd * sg.nchunk <= kFusedReduce &&
+                     int64_t(m) * nd * sg.nseg <= kFusedOutputs && sg.ticket && threads >= 32;
   GivensArgs none;
   const GivensArgs& g = gv && fused ? *gv : none;
   auto go = [&](auto kern) {
