@@ -130,8 +130,8 @@ int far_nchunks(int64_t ntarg, int64_t nptso, int kind, int precision, int nd, i
 // chunks that fills `waves` waves of resident blocks.
 // md = 1 selects the multi-density kernel's shapes (nd > 1).
 int far_variants();
-constexpr int kFarSmall = 5;  // one-density shape for few targets
-bool far_small_fits(int64_t ntarg, int nd);  // whether the autotuner tries it
+constexpr int kFarSmall = 5;  // shape for few targets: one density, or 2 to 8 in FP32 Laplace
+bool far_small_fits(int64_t ntarg, int kind, int precision, int nd);  // the autotuner tries it
 // Matrix-instruction far field (variants 3 and 4 of the multi-density
 // Helmholtz path; FP32 far_tc.cu, FP64 far_dmma.cu): densities per CTA, 0
 // where the variant does not apply.

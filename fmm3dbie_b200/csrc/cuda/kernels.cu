@@ -878,13 +878,14 @@ __device__ __forceinline__ void far_md_lap_block(const Geometry& g, const KParam
   }
 }
 
-template <int KIND, typename R, int NT, int TPT, int MD, int TILE, bool CK>
+template <int KIND, typename R, int NT, int TPT, int MD, int TILE, bool CK,
+          bool PAIRS = kMdLap32<KIND, R, MD>>
 __global__ void __launch_bounds__(NT) far_md_kernel(Geometry g, KParams kp,
                                                     const R* __restrict__ ab,
                                                     const R* __restrict__ sig, int nd,
                                                     double* __restrict__ partial,
                                                     int64_t chunk_len) {
-  if constexpr (kMdLap32<KIND, R, MD>) {
+  if constexpr (PAIRS) {
     __shared__ float4 tile[TILE * kMdLapWords<MD>];
     far_md_lap_block<NT, TPT, MD, TILE>(g, kp, ab, sig, nd, partial, chunk_len, blockIdx.x,
                                         blockIdx.y, blockIdx.z, tile);
@@ -2288,9 +2289,12 @@ cudaError_t far_dispatch(const Geometry& g, const KParams& kp, const MatvecArgs&
   return launch_far_t<KIND, R, NT, TPT, CK>(g, kp, a, st);
 }
 
-// The autotuner tries the small-problem shape up to this many targets: at 2,400
-// it wins in FP32 (23.4 against 27.3 us, Helmholtz) and loses in FP64 (54
-// against 50), at 5,400 it loses everywhere.
+// The autotuner tries the small-problem shapes up to this many targets.  One
+// density: at 2,400 far_small_kernel wins in FP32 (23.4 against 27.3 us,
+// Helmholtz) and loses in FP64 (54 against 50), at 5,400 it loses everywhere.
+// FP32 Laplace, 8 densities: far_md_small 11.0 against the pairs' 13.6 us at 864
+// targets, 19.6 against 23.3 at 2,400, 38.9 against 39.9 at 3,750, 72.6 against
+// 72.7 at 5,400; 2 and 4 densities win up to 864 only.
 constexpr int64_t kSmallMax = 4096;
 
 template <int KIND, typename R, bool CK>
@@ -2366,6 +2370,28 @@ cudaError_t far_md_dispatch(const Geometry& g, const KParams& kp, const MatvecAr
   return cudaGetLastError();
 }
 
+// FP32 Laplace blocks of up to 8 densities for few targets: one target a thread
+// without pairs, which leaves twice the blocks of the paired shapes.
+template <int CL>
+cudaError_t far_md_small(const Geometry& g, const KParams& kp, const MatvecArgs& a, cudaStream_t st,
+                         int* occ) {
+  constexpr int NT = kMdShapes[CL][0][0], MD = kMdShapes[CL][0][2];
+  auto kern = far_md_kernel<0, float, NT, 1, MD, kFarTile, false, false>;
+  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, NT, 0);
+  const int64_t tblocks = (g.ntarg + NT - 1) / NT;
+  int64_t chunk = (g.nptso + a.nchunks - 1) / a.nchunks;
+  chunk = ((chunk + kFarTile - 1) / kFarTile) * kFarTile;
+  kern<<<dim3(unsigned(tblocks), unsigned(a.nchunks), unsigned((a.nd + MD - 1) / MD)), NT, 0, st>>>(
+      g, kp, static_cast<const float*>(a.ab), static_cast<const float*>(a.strengths), a.nd,
+      a.partial, chunk);
+  return cudaGetLastError();
+}
+
+// Whether nd densities have that shape.
+bool md_small_shape(int kind, int precision, int nd) {
+  return kind == 0 && precision == 1 && nd > 1 && nd <= 8;
+}
+
 template <int KIND, typename R, bool CK, int CL>
 cudaError_t far_md_class(int v, const Geometry& g, const KParams& kp, const MatvecArgs& a,
                          cudaStream_t st, int* occ) {
@@ -2398,6 +2424,9 @@ cudaError_t far_md_any(const Geometry& g, const KParams& kp, const MatvecArgs& a
   int v = a.far_variant;
   if (v >= 3) {
     if (far_tc_group(v, a.nd, a.precision, kp.kind) > 0) return far_tc(v, g, kp, a, st, occ);
+    if (v == kFarSmall && md_small_shape(kp.kind, a.precision, a.nd))
+      return md_class(a.nd) == 0 ? far_md_small<0>(g, kp, a, st, occ)
+                                 : far_md_small<1>(g, kp, a, st, occ);
     if (occ) {  // not a shape of this path: the autotuner skips it
       *occ = 0;
       return cudaSuccess;
@@ -2787,12 +2816,16 @@ cudaError_t launch_source_consts(const Geometry& g, const KParams& kp, int preci
 
 int far_variants() { return kFarSmall + 1; }
 
-bool far_small_fits(int64_t ntarg, int nd) { return nd == 1 && ntarg <= kSmallMax; }
+bool far_small_fits(int64_t ntarg, int kind, int precision, int nd) {
+  return (nd == 1 || md_small_shape(kind, precision, nd)) && ntarg <= kSmallMax;
+}
 
 int far_block_targets(int kind, int precision, int variant, int md, int nd) {
   if (md && far_tc_group(variant, nd, precision, kind) > 0) return far_tc_targets(precision);
   if (!md && variant == kFarSmall) return kSmallTargets;
   const int v = variant < 0 || variant > 2 ? 0 : variant;
+  if (md && variant == kFarSmall && md_small_shape(kind, precision, nd))
+    return kMdShapes[md_class(nd)][0][0];
   if (md) return kMdShapes[md_class(nd)][v][0] * md_tpt(kind, precision, md_class(nd), v);
   return precision == 1 ? kF32Shapes[v][0] * kF32Shapes[v][1]
                         : kF64Shapes[v][0] * kF64Shapes[v][1];

@@ -840,7 +840,7 @@ int Plan::tune_far(int precision, int nd, dev::MatvecArgs& a, cudaStream_t st, F
     const int md = nd > 1;
     const bool tc = precision == 0 || tc_room();
     for (int v = 0; v < dev::far_variants(); ++v) {
-      if (v == dev::kFarSmall && !dev::far_small_fits(ntarg, nd)) continue;
+      if (v == dev::kFarSmall && !dev::far_small_fits(ntarg, kind, precision, nd)) continue;
       if (!tc && md && dev::far_tc_group(v, nd, precision, kind) > 0) {
         all_shapes = false;
         continue;
